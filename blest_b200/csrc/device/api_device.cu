@@ -150,7 +150,7 @@ void workspace_alloc(const blest_graph* g, Workspace& w) {
     alloc((void**)&w.counters, sizeof(dev::RunCounters));
     alloc((void**)&w.levels, 4ull * n);
     alloc((void**)&w.parents, 4ull * n);
-    alloc((void**)&w.labels_old, 4ull * n);
+    alloc((void**)&w.cc_parent, 8ull * n);
     alloc((void**)&w.trace, sizeof(blest_level_trace) * BLEST_TRACE_CAPACITY);
     summary_geometry(w.words, w.sum_shift, w.sum_words);
     for (int i = 0; i < 3; ++i) alloc((void**)&w.summary[i], 4ull * w.sum_words);
@@ -173,7 +173,7 @@ void workspace_free(Workspace& w) {
     cudaFree(w.counters);
     cudaFree(w.levels);
     cudaFree(w.parents);
-    cudaFree(w.labels_old);
+    cudaFree(w.cc_parent);
     cudaFree(w.trace);
     for (auto& x : w.summary) cudaFree(x);
     cudaFree(w.heavy);
@@ -359,7 +359,9 @@ void attach_tiles(blest_graph* g, const uint32_t* rows, const uint32_t* masks, c
 // The pull side of a resident graph: CSR lists ordered by descending
 // neighbour degree, the has-in-neighbour bitmap and the long-list pieces;
 // then the graph's stream and default workspace.
-void graph_attach_csr(blest_graph* g, const blest_csr_view* csr) {
+// `symmetric`: the caller knows that the tiles' edges are symmetric and the
+// same as the lists'; otherwise that is checked on the device.
+void graph_attach_csr(blest_graph* g, const blest_csr_view* csr, bool symmetric) {
     blest::dev::DevGraph& d = g->d;
     d.nnz = csr->nnz;
     d.degree_total = csr->nnz;
@@ -375,7 +377,8 @@ void graph_attach_csr(blest_graph* g, const blest_csr_view* csr) {
 #pragma omp parallel for schedule(dynamic, 1024)
         for (int64_t u = 0; u < (int64_t)csr->n; ++u) {
             std::stable_sort(ids.begin() + rp[u], ids.begin() + rp[u + 1], [rp](uint32_t x, uint32_t y) {
-                return rp[x + 1] - rp[x] > rp[y + 1] - rp[y];
+                const uint32_t dx = rp[x + 1] - rp[x], dy = rp[y + 1] - rp[y];
+                return dx != dy ? dx > dy : x < y;
             });
         }
         d.csr_ids = blest::upload(g, ids.data(), ids.size());
@@ -397,6 +400,7 @@ void graph_attach_csr(blest_graph* g, const blest_csr_view* csr) {
         d.pull_chunks = blest::upload(g, chunks.data(), chunks.size());
     }
     g->undirected_edges = csr->nnz / 2;
+    g->symmetric = symmetric || blest::tiles_symmetric_device(d, nullptr);
     BLEST_CUDA(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
     g->owns_stream = true;
     g->default_ws = new blest_workspace;
@@ -451,7 +455,7 @@ int blest_graph_create(const blest_bvss_view* bvss, const blest_csr_view* csr, b
             release();
             (void)d;
         }
-        graph_attach_csr(g, csr);
+        graph_attach_csr(g, csr, false);
         *out = g;
     });
     if (rc != BLEST_OK && g) blest_graph_destroy(g);
@@ -486,7 +490,7 @@ int blest_graph_create_from_csc(const blest_csc* csc, const blest_csc* csr, int 
             throw;
         }
         blest::device_bvss_free(b);
-        graph_attach_csr(g, &cv);
+        graph_attach_csr(g, &cv, csr == nullptr);  // without a CSR: checked above
         *out = g;
     });
     if (rc != BLEST_OK && g) blest_graph_destroy(g);

@@ -289,6 +289,58 @@ __global__ void rset_tile_kernel(const uint64_t* slice_off, uint32_t R, uint32_t
         rset_tile[r] = (uint32_t)(slice_off[r] / 4);
 }
 
+// Position of x in list v of the pull lists (sorted by descending list
+// length, ties by id), or nnz when it is not there.
+__device__ __forceinline__ uint32_t find_in_list(const uint32_t* ptrs, const uint32_t* ids, uint32_t nnz, uint32_t v,
+                                                 uint32_t x) {
+    uint32_t lo = __ldg(&ptrs[v]);
+    const uint32_t end = __ldg(&ptrs[v + 1]);
+    const uint32_t dx = __ldg(&ptrs[x + 1]) - __ldg(&ptrs[x]);
+    uint32_t hi = end;
+    while (lo < hi) {
+        const uint32_t mid = lo + (hi - lo) / 2;
+        const uint32_t y = __ldg(&ids[mid]);
+        const uint32_t dy = __ldg(&ptrs[y + 1]) - __ldg(&ptrs[y]);
+        if (dy > dx || (dy == dx && y < x)) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo < end && __ldg(&ids[lo]) == x ? lo : nnz;
+}
+
+// Looks every edge c -> r of the tiles up in list c (marking its position)
+// and in list r. A miss or a position met twice sets *bad; *edges counts the
+// edges. With *bad == 0 and *edges == nnz the lists hold exactly the tiles'
+// edges, each once, and the edges are symmetric. Bound by dependent L2 and
+// DRAM reads of the two searches; a directed graph stops at its first miss.
+__global__ void tiles_symmetric_kernel(DevGraph g, uint32_t* seen, uint32_t* bad, unsigned long long* edges) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+    uint64_t count = 0;
+    for (uint32_t r = warp; r < g.no_real; r += nwarps) {
+        if (*(volatile uint32_t*)bad) break;
+        const uint32_t t1 = __ldg(&g.rset_tile[r + 1]);
+        for (uint32_t t = __ldg(&g.rset_tile[r]) + lane; t < t1; t += 32) {
+            const uint4 rows = __ldg(&g.row4[t]);
+            const uint32_t mask = __ldg(&g.masks[t]);
+            const uint32_t rowk[4] = {rows.x, rows.y, rows.z, rows.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                for (uint32_t m = (mask >> (8 * k)) & 0xFFu; m; m &= m - 1) {
+                    const uint32_t c = r * 8 + __ffs(m) - 1, row = rowk[k];
+                    const uint32_t at = find_in_list(g.csr_ptrs, g.csr_ids, g.nnz, c, row);
+                    bool ok = at < g.nnz && find_in_list(g.csr_ptrs, g.csr_ids, g.nnz, row, c) < g.nnz;
+                    if (ok) ok = !((atomicOr(&seen[at >> 5], 1u << (at & 31)) >> (at & 31)) & 1u);
+                    if (!ok) *(volatile uint32_t*)bad = 1u;
+                    ++count;
+                }
+            }
+        }
+        __syncwarp();
+    }
+    for (int d = 16; d > 0; d >>= 1) count += __shfl_xor_sync(0xFFFFFFFFu, count, d);
+    if (lane == 0 && count) atomicAdd(edges, (unsigned long long)count);
+}
+
 }  // namespace dev
 
 namespace {
@@ -427,6 +479,27 @@ void compact_tiles_device(const uint32_t* row_ids, const uint32_t* masks, const 
         out = CompactTiles{};
         throw;
     }
+}
+
+bool tiles_symmetric_device(const dev::DevGraph& d, cudaStream_t s) {
+    int dev = 0, sms = 0;
+    BLEST_CUDA(cudaGetDevice(&dev));
+    BLEST_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    struct Out {
+        unsigned long long edges;
+        uint32_t bad, pad;
+    } h{};
+    Scratch tmp;
+    const size_t words = ((size_t)d.nnz + 31) / 32 + 1;
+    uint32_t* seen = tmp.get<uint32_t>(words);
+    Out* out = tmp.get<Out>(1);
+    BLEST_CUDA(cudaMemsetAsync(seen, 0, 4 * words, s));
+    BLEST_CUDA(cudaMemsetAsync(out, 0, sizeof(Out), s));
+    dev::tiles_symmetric_kernel<<<sms * 8, 256, 0, s>>>(d, seen, &out->bad, &out->edges);
+    BLEST_CUDA(cudaGetLastError());
+    BLEST_CUDA(cudaMemcpyAsync(&h, out, sizeof(Out), cudaMemcpyDeviceToHost, s));
+    BLEST_CUDA(cudaStreamSynchronize(s));
+    return !h.bad && h.edges == d.nnz;
 }
 
 void device_bvss_free(DeviceBvss& b) {

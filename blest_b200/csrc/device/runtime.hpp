@@ -31,7 +31,7 @@ struct Workspace {
     dev::RunCounters* counters = nullptr;
     uint32_t* levels = nullptr;   // internal output buffers (host-output calls)
     uint32_t* parents = nullptr;
-    uint32_t* labels_old = nullptr;  // CC
+    uint32_t* cc_parent = nullptr;  // CC: union-find parents and kept edges, n words each
     dev::RunCounters* host_counters = nullptr;  // pinned mirror
     blest_level_trace* trace = nullptr;         // device, BLEST_TRACE_CAPACITY records
     uint32_t* summary[3] = {nullptr, nullptr, nullptr};  // frontier summaries
@@ -70,6 +70,9 @@ struct blest_graph {
     std::vector<void*> allocations;
     uint64_t graph_bytes = 0;
     uint64_t undirected_edges = 0;
+    // Every edge u -> v of the tiles has its v -> u, and the pull lists hold
+    // exactly the same edges (checked edge by edge when the graph is made).
+    bool symmetric = false;
     cudaStream_t stream = nullptr;
     bool owns_stream = false;
     blest_workspace* default_ws = nullptr;
@@ -146,6 +149,10 @@ struct CompactTiles {
 };
 void compact_tiles_device(const uint32_t* row_ids, const uint32_t* masks, const uint32_t* rset_tile, uint32_t R,
                           cudaStream_t s, CompactTiles& out);
+// True when the tiles' edge relation is symmetric and the pull lists (each
+// sorted by descending list length, ties by id) hold exactly its edges, each
+// once. Blocking; every edge is looked up, nothing is sampled or hashed.
+bool tiles_symmetric_device(const dev::DevGraph& d, cudaStream_t s);
 void mbfs_scratch_free(void* p);
 // Allocate the multi-source BFS state of `words` 32-bit words per vertex now.
 void mbfs_reserve(Workspace& w, uint32_t n, uint32_t words);
