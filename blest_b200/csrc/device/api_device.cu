@@ -154,6 +154,7 @@ void workspace_alloc(const blest_graph* g, Workspace& w) {
     alloc((void**)&w.trace, sizeof(blest_level_trace) * BLEST_TRACE_CAPACITY);
     summary_geometry(w.words, w.sum_shift, w.sum_words);
     for (int i = 0; i < 3; ++i) alloc((void**)&w.summary[i], 4ull * w.sum_words);
+    if (g->d.out_ptrs) alloc((void**)&w.pieces, sizeof(uint4) * (size_t)g->d.piece_cap);
     w.heavy_cap = g->d.nnz / 1024 + 64;
     alloc((void**)&w.heavy, sizeof(uint4) * w.heavy_cap);
     BLEST_CUDA(cudaMallocHost((void**)&w.host_counters, sizeof(dev::RunCounters)));
@@ -176,6 +177,7 @@ void workspace_free(Workspace& w) {
     cudaFree(w.cc_parent);
     cudaFree(w.trace);
     for (auto& x : w.summary) cudaFree(x);
+    cudaFree(w.pieces);
     cudaFree(w.heavy);
     mbfs_scratch_free(w.mbfs);
     if (w.records) cudaFreeHost(w.records);
@@ -401,6 +403,20 @@ void graph_attach_csr(blest_graph* g, const blest_csr_view* csr, bool symmetric)
     }
     g->undirected_edges = csr->nnz / 2;
     g->symmetric = symmetric || blest::tiles_symmetric_device(d, nullptr);
+    uint64_t out_edges = d.nnz;
+    blest::OutLists out;
+    if (g->symmetric) {
+        d.out_ptrs = d.csr_ptrs;
+        d.out_ids = d.csr_ids;
+    } else if (blest::out_lists_device(d, nullptr, out)) {
+        g->allocations.push_back(out.ptrs);
+        g->allocations.push_back(out.ids);
+        g->graph_bytes += 4ull * (csr->n + 1ull) + 4ull * out.edges;
+        d.out_ptrs = out.ptrs;
+        d.out_ids = out.ids;
+        out_edges = out.edges;
+    }
+    d.piece_cap = (uint32_t)(csr->n + out_edges / blest::dev::kBfsPieceEdges + 64);
     BLEST_CUDA(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
     g->owns_stream = true;
     g->default_ws = new blest_workspace;

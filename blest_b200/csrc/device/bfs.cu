@@ -1,5 +1,8 @@
 // Single-source direction-optimising BFS over BVSS tiles (push) and CSR
-// in-neighbour lists (pull), as ONE persistent cooperative kernel per BFS.
+// in-neighbour lists (pull), as ONE persistent cooperative kernel per BFS: the
+// kernel of the b1-MMA slice test and of blest_bfs_noalloc, whose callers
+// hand over tiles and no out-lists. Every other call pushes over out-lists
+// (bfs_lists.cu), which is faster at every size measured there.
 //
 // Replaces the six BFS kernels of BFS/BVSSBFSKernel.cuh (:33-1261) and the
 // launcher BVSSBFSKernel::hostCode (:1283-1608). Results are the same
@@ -26,6 +29,7 @@
 #include <tuple>
 #include <string>
 
+#include "bfs_args.cuh"
 #include "common.cuh"
 #include "runtime.hpp"
 #include "../host/common.hpp"
@@ -33,42 +37,6 @@
 
 namespace blest {
 namespace dev {
-
-struct BfsArgs {
-    DevGraph g;
-    uint32_t* levels;
-    uint32_t* parents;
-    uint32_t* visited;
-    uint32_t* frontier0;
-    uint32_t* frontier1;
-    uint32_t* frontier2;
-    uint32_t* q_rset;
-    uint32_t* q_off;
-    RunCounters* ctr;
-    uint32_t words;
-    uint32_t src;
-    int direction;
-    float alpha;
-    float beta;
-    blest_level_trace* trace;  // optional per-level records
-    // Frontier summary per level (1 bit per 2^sum_shift frontier words),
-    // staged in shared memory by the pull phase to skip empty words.
-    uint32_t* summary0;
-    uint32_t* summary1;
-    uint32_t* summary2;
-    uint32_t sum_shift;
-    uint32_t sum_words;
-    // Pull: unvisited vertices whose remaining list is longer than
-    // heavy_min are scanned by all warps in kHeavyChunk pieces after a
-    // mid-level barrier. heavy: {vertex, first, end, chunk offset} records.
-    uint4* heavy;
-    uint32_t heavy_cap;
-    uint32_t heavy_min;
-    // Where the run's outcome goes (null: nowhere) and the call number it
-    // carries.
-    RunRecord* record;
-    uint64_t seq;
-};
 
 __device__ __forceinline__ uint32_t* summary_buf(const BfsArgs& a, uint32_t level) {
     const uint32_t m = level % 3;
@@ -79,14 +47,6 @@ __device__ __forceinline__ void summary_set(const BfsArgs& a, uint32_t* sum, uin
     const uint32_t sb = word >> a.sum_shift;
     atomicOr(&sum[sb >> 5], 1u << (sb & 31));
 }
-
-// Neighbours a lane scans alone in the pull phase before the warp takes over,
-// and how many of them it has in flight at once (a warp waits for its
-// slowest lane, so fewer, wider rounds finish sooner).
-constexpr uint32_t kPullLaneScan = 32;
-constexpr uint32_t kPullUnroll = 4;
-// Neighbours per piece of a heavy (very long) in-neighbour list.
-constexpr uint32_t kHeavyChunk = 256;
 
 __device__ __forceinline__ uint32_t* frontier_buf(const BfsArgs& a, uint32_t level) {
     const uint32_t m = level % 3;
@@ -963,22 +923,7 @@ template <bool ALIGNED, bool MMA, bool PARENTS>
 __global__ void __launch_bounds__(512, 2) bfs_persistent_kernel(BfsArgs a) {
     const uint64_t t0 = global_ns();
     bfs_run<ALIGNED, MMA, PARENTS>(a);
-    if (a.record && blockIdx.x == 0 && threadIdx.x == 0) {
-        const RunCounters* c = a.ctr;
-        RunRecord* r = a.record;
-        r->start_ns = t0;
-        r->end_ns = global_ns();
-        r->error = ld_relaxed(&c->error);
-        r->discovered = c->discovered;
-        r->degree = c->degree;
-        r->levels = c->levels;
-        r->push_levels = c->push_levels;
-        r->pull_levels = c->pull_levels;
-        r->source = a.src;
-        // the host polls seq: it must become visible after the rest
-        __threadfence_system();
-        *(volatile unsigned long long*)&r->seq = a.seq;
-    }
+    write_record(a, t0);
 }
 
 }  // namespace dev
@@ -1051,6 +996,11 @@ void launch_bfs(const blest_graph* g, Workspace& w, uint32_t src, uint32_t* leve
     const int threads = p.threads_per_block > 0 ? p.threads_per_block : 512;
     if (threads % 32 || threads > 512) throw Error(BLEST_ERR_INVALID_ARG, "threads_per_block must be a multiple of 32, <= 512");
     const bool mma = p.slice_test == BLEST_TEST_B1_MMA;
+    if (!mma && g->d.out_ptrs) {
+        a.pieces = w.pieces;
+        launch_bfs_lists(g, a, p.blocks_per_sm, threads, w.grid_blocks, s);
+        return;
+    }
     const bool par = parents != nullptr;
     if (mma) {
         if (par) launch_variant<true, true, true>(g, a, p.blocks_per_sm, threads, w.grid_blocks, s);

@@ -1,0 +1,1032 @@
+// Single-source direction-optimising BFS over adjacency lists, as ONE
+// persistent cooperative kernel per BFS: the default kernel behind blest_bfs
+// and blest_bfs_ws (bfs.cu keeps the kernel over BVSS tiles for the b1-MMA
+// slice test and for blest_bfs_noalloc, whose callers hand over tiles only).
+//
+// Same levels as the six BFS kernels of BFS/BVSSBFSKernel.cuh (:33-1261). A
+// push level over tiles reads every slice of every set that holds one
+// frontier vertex (a uniform graph's level of 41 k vertices: 49 MB of tiles
+// for 1.3 M edges, 62 us); here it reads the frontier's own out-lists.
+//
+// The frontier has two forms, and each level uses the one its direction
+// reads:
+//  - two queues of {first edge, edges, vertex} (push): lists of at most 128
+//    edges, of which a warp takes 32 and walks their edges as one flat range,
+//    and longer ones, whose 128-edge pieces are numbered through (each entry
+//    holds its first piece's number) and split evenly over the warps. One
+//    entry per vertex: writing out the pieces themselves took 24 us for the
+//    317 k pieces of RMAT-22's second level, its edges 7 us;
+//  - a bitmap with a summary of its non-empty words (pull, and the result of
+//    a lazy push).
+// A change of form costs one more grid barrier, once or twice in a run; in
+// return push levels keep no bitmap and pull levels queue nothing.
+//
+// What bounds it: levels are short, so chains of dependent L2 round trips
+// (~0.7 us each) and words that every warp updates (about one access a
+// nanosecond per word). A block therefore gathers its level's discoveries in
+// shared memory and appends them with one atomic, and while the frontier is
+// small ("solo" levels) block 0 runs the levels alone out of shared memory,
+// with block barriers only, while the others wait in one grid barrier.
+// Against the kernel over tiles (a whole call): RMAT 2^10 63 -> 49 us, RMAT-16
+// 72 -> 64, RMAT-22 215 -> 158 a BFS, grid 2901 x 2801 3080 -> 1200 (widest
+// level, 306 k vertices: 71 -> 24; smallest levels 8 -> 3), uniform 2 M
+// vertices x degree 32 211 -> 137 (41 k-vertex level 62 -> 28).
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <map>
+#include <mutex>
+#include <tuple>
+
+#include "../host/common.hpp"
+#include "../host/errors.hpp"
+#include "bfs_args.cuh"
+#include "common.cuh"
+#include "runtime.hpp"
+
+namespace blest {
+namespace dev {
+namespace {
+
+constexpr uint32_t kPiece = kBfsPieceEdges;
+constexpr uint32_t kMaxWarps = 16;      // per block (512 threads)
+constexpr uint32_t kWinners = 2048;     // discoveries a block gathers before it appends one warp at a time
+// A level is run by block 0 alone when its pieces and edges fit these: one
+// flat step of its warps (16 warps x 128 edges).
+constexpr uint32_t kSoloPieces = 512;
+constexpr uint32_t kSoloEdges = 2048;
+// Solo levels in a row, after which the waiting blocks' barrier is renewed
+// (its wait is bounded, a solo level takes a few microseconds).
+constexpr uint32_t kSoloLevels = 512;
+
+// A queue position or size: short lists, long lists, pieces of the long lists.
+struct Span {
+    uint32_t a, b, u;
+};
+
+struct BlockState {
+    uint32_t win_v[kWinners], win_b[kWinners], win_d[kWinners];  // vertex, first out-edge, out-degree
+    uint4 solo[kSoloPieces];
+    uint32_t found[32 * kMaxWarps];  // pull: found bits of a warp's 32 words
+    uint32_t win_cnt, win_end;       // appended; where the first append that did not fit starts
+    uint32_t tot_ab[kMaxWarps], tot_u[kMaxWarps], tot_d[kMaxWarps], tot_disc[kMaxWarps], tot_deg[kMaxWarps];
+    Span base;
+    uint32_t ok;
+    unsigned long long val[kSlotWords];  // the step's counters after its barrier
+};
+
+// The run's state, the same in every block.
+struct Run {
+    uint32_t level;
+    uint32_t step;        // rounds of the main loop: counter slot (step % 3), record of the solo levels (step % 2)
+    Span from, size;      // the frontier's entries in the two queues (from.u is unused)
+    uint32_t D2, D1;      // vertices discovered up to the last level but one / the last level
+    uint32_t nf_prev;
+    unsigned long long G2, G1;  // their degree sums
+};
+
+__device__ __forceinline__ uint32_t* bitmap_of(const BfsArgs& a, uint32_t gen) {
+    const uint32_t m = gen % 3;
+    return m == 0 ? a.frontier0 : (m == 1 ? a.frontier1 : a.frontier2);
+}
+
+__device__ __forceinline__ uint32_t* summary_of(const BfsArgs& a, uint32_t gen) {
+    const uint32_t m = gen % 3;
+    return m == 0 ? a.summary0 : (m == 1 ? a.summary1 : a.summary2);
+}
+
+__device__ __forceinline__ void mark_summary(const BfsArgs& a, uint32_t* sum, uint32_t word) {
+    const uint32_t sb = word >> a.sum_shift;
+    atomicOr(&sum[sb >> 5], 1u << (sb & 31));
+}
+
+__device__ __forceinline__ uint32_t pieces_of(uint32_t degree) { return (degree + kPiece - 1) / kPiece; }
+
+// Where a step appends: entries from `from` on, counted by *ca (short lists)
+// and *cb (long lists, packed entries << kQShift | pieces), which start at 0.
+struct Tail {
+    Span from;
+    unsigned long long* ca;
+    unsigned long long* cb;
+};
+
+__device__ __forceinline__ Span span_of(unsigned long long ca, unsigned long long cb) {
+    return Span{(uint32_t)ca, (uint32_t)(cb >> kQShift), (uint32_t)(cb & kQUnitMask)};
+}
+
+// Reserve room for `need` entries (one thread); returns where they go.
+__device__ __forceinline__ Span reserve(const Tail& t, const Span& need) {
+    Span at{0u, 0u, 0u};
+    if (need.a) at.a = t.from.a + (uint32_t)atomicAdd(t.ca, (unsigned long long)need.a);
+    if (need.b) {
+        const unsigned long long o = atomicAdd(t.cb, ((unsigned long long)need.b << kQShift) | need.u);
+        at.b = t.from.b + (uint32_t)(o >> kQShift);
+        at.u = (uint32_t)(o & kQUnitMask);
+    }
+    return at;
+}
+
+// Write vertex v's entry and advance `at` past it. Every vertex is queued at
+// most once, so the queues cannot overflow.
+__device__ __forceinline__ void put_entry(const BfsArgs& a, Span& at, uint32_t v, uint32_t b, uint32_t d) {
+    if (d == 0) return;
+    const bool is_long = d > kPiece;
+    const uint32_t e = is_long ? a.g.n + at.b : at.a;
+    if (is_long ? e < a.g.piece_cap : e < a.g.n) a.pieces[e] = make_uint4(b, d, v, is_long ? at.u : 0u);
+    else set_error(a.ctr, BLEST_ERR_DEVICE_INDEX);
+    if (is_long) {
+        ++at.b;
+        at.u += pieces_of(d);
+    } else {
+        ++at.a;
+    }
+}
+
+__device__ __forceinline__ uint32_t warp_incl(uint32_t x) {
+    const uint32_t lane = threadIdx.x & 31;
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+        const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, x, s);
+        if (lane >= s) x += o;
+    }
+    return x;
+}
+
+// Hand a warp's discoveries (bit k of `won`: vertex v[k], out-list at b[k] of
+// length d[k]) to the block's buffer; when it is full, to the global queues.
+__device__ __forceinline__ void emit(const BfsArgs& a, BlockState& B, const uint32_t (&v)[4], const uint32_t (&b)[4],
+                                     const uint32_t (&d)[4], uint32_t won, const Tail& tail) {
+    const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1u;
+    uint32_t off[4], total = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, (won >> k) & 1u);
+        off[k] = total + __popc(m & below);
+        total += __popc(m);
+    }
+    if (!total) return;
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(&B.win_cnt, total);
+    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    if (base + total <= kWinners) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (!((won >> k) & 1u)) continue;
+            B.win_v[base + off[k]] = v[k];
+            B.win_b[base + off[k]] = b[k];
+            B.win_d[base + off[k]] = d[k];
+        }
+        return;
+    }
+    // the counter only grows, so every later append fails too and the entries
+    // before the first failed one are exactly those written
+    if (lane == 0) atomicMin(&B.win_end, base);
+    uint32_t ab = 0, u = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (!((won >> k) & 1u) || !d[k]) continue;
+        ab += d[k] > kPiece ? 0x10000u : 1u;
+        u += d[k] > kPiece ? pieces_of(d[k]) : 0u;
+    }
+    const uint32_t iab = warp_incl(ab), iu = warp_incl(u);
+    Span at{0u, 0u, 0u};
+    if (lane == 31) at = reserve(tail, Span{iab & 0xFFFFu, iab >> 16, iu});
+    at.a = __shfl_sync(0xFFFFFFFFu, at.a, 31) + ((iab - ab) & 0xFFFFu);
+    at.b = __shfl_sync(0xFFFFFFFFu, at.b, 31) + ((iab - ab) >> 16);
+    at.u = __shfl_sync(0xFFFFFFFFu, at.u, 31) + iu - u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if ((won >> k) & 1u) put_entry(a, at, v[k], b[k], d[k]);
+}
+
+// The block's buffered discoveries as queue entries: into the global queues
+// (one reservation per block), or, when `solo` and they fit, as pieces into
+// B.solo. Adds the block's discovery count and degree sum to lvl[1], lvl[2]
+// (when lvl).
+struct Flushed {
+    uint32_t pieces, disc, deg;
+    bool in_solo;
+};
+__device__ __forceinline__ Flushed flush(const BfsArgs& a, BlockState& B, const Tail& tail, unsigned long long* lvl,
+                                         uint32_t disc, uint32_t deg, bool solo) {
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    __syncthreads();
+    const uint32_t m = min(B.win_cnt, B.win_end);
+    const bool spilled = B.win_end != kWinners;
+    uint32_t ab = 0, u = 0, ed = 0;  // short | long << 16 entries, pieces of the long ones, edges
+    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
+        const uint32_t d = B.win_d[i];
+        ab += d > kPiece ? 0x10000u : (d ? 1u : 0u);
+        u += d > kPiece ? pieces_of(d) : 0u;
+        ed += d;
+    }
+    const uint32_t iab = warp_incl(ab), iu = warp_incl(u);
+    ed = __reduce_add_sync(0xFFFFFFFFu, ed);
+    disc = __reduce_add_sync(0xFFFFFFFFu, disc);
+    deg = __reduce_add_sync(0xFFFFFFFFu, deg);
+    if (lane == 31) {
+        B.tot_ab[w] = iab;
+        B.tot_u[w] = iu;
+        B.tot_d[w] = ed;
+        B.tot_disc[w] = disc;
+        B.tot_deg[w] = deg;
+    }
+    __syncthreads();
+    Flushed F{0, 0, 0, false};
+    uint32_t before_ab = 0, before_u = 0, all_ab = 0, all_u = 0, edges = 0;
+    for (uint32_t i = 0; i < nw; ++i) {
+        if (i == w) {
+            before_ab = all_ab;
+            before_u = all_u;
+        }
+        all_ab += B.tot_ab[i];
+        all_u += B.tot_u[i];
+        edges += B.tot_d[i];
+        F.disc += B.tot_disc[i];
+        F.deg += B.tot_deg[i];
+    }
+    F.pieces = (all_ab & 0xFFFFu) + all_u;
+    F.in_solo = solo && !spilled && F.pieces <= kSoloPieces && edges <= kSoloEdges;
+    if (threadIdx.x == 0) {
+        if (lvl && F.disc) {
+            atomicAdd(&lvl[1], (unsigned long long)F.disc);
+            atomicAdd(&lvl[2], (unsigned long long)F.deg);
+        }
+        if (!F.in_solo) B.base = reserve(tail, Span{all_ab & 0xFFFFu, all_ab >> 16, all_u});
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        B.win_cnt = 0;
+        B.win_end = kWinners;
+    }
+    const uint32_t pab = before_ab + iab - ab, pu = before_u + iu - u;
+    if (F.in_solo) {
+        uint32_t at = (pab & 0xFFFFu) + pu;
+        for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
+            const uint32_t b = B.win_b[i], d = B.win_d[i], v = B.win_v[i];
+            for (uint32_t k = 0; k < d; k += kPiece) B.solo[at++] = make_uint4(b + k, min(kPiece, d - k), v, 0u);
+        }
+    } else {
+        Span at{B.base.a + (pab & 0xFFFFu), B.base.b + (pab >> 16), B.base.u + pu};
+        for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) put_entry(a, at, B.win_v[i], B.win_b[i], B.win_d[i]);
+    }
+    return F;
+}
+
+// The out-edges of the pieces that a warp's lanes hold (p.y = 0: none): each
+// unvisited end is claimed by its bit in `visited` and recorded, or, in a lazy
+// level, only marked in fcur (the sweep drops what was visited).
+template <bool PARENTS, bool LAZY>
+__device__ __forceinline__ void push_batch(const BfsArgs& a, BlockState& B, const uint4& p, uint32_t level,
+                                           bool precheck, uint32_t* fcur, const Tail& tail, uint32_t& disc,
+                                           uint32_t& deg) {
+    const uint32_t lane = threadIdx.x & 31;
+    const DevGraph& g = a.g;
+    const bool own_lists = g.out_ptrs != g.csr_ptrs;  // directed: degrees are counted over the in-lists
+    const uint32_t incl = warp_incl(p.y);
+    const uint32_t off = incl - p.y;
+    const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    const uint32_t from = p.x - off;  // edge of flat index i in this piece: from + i
+    for (uint32_t base = 0; base < total; base += 128) {
+        uint32_t row[4], src[4], live = 0;
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u) {
+            const uint32_t i = base + u * 32 + lane;
+            uint32_t lo = 0;
+#pragma unroll
+            for (uint32_t st = 16; st > 0; st >>= 1) {
+                const uint32_t o = __shfl_sync(0xFFFFFFFFu, off, lo + st);  // lo + st <= 31
+                if (o <= i) lo += st;
+            }
+            const uint32_t f = __shfl_sync(0xFFFFFFFFu, from, lo);
+            src[u] = PARENTS ? __shfl_sync(0xFFFFFFFFu, p.z, lo) : 0u;
+            row[u] = i < total ? __ldg(&g.out_ids[f + i]) : kUnreached;
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u) live |= (row[u] < g.n ? 1u : 0u) << u;
+        if (precheck) {
+            uint32_t vis[4];
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u) vis[u] = (live >> u) & 1u ? __ldcg(&a.visited[row[u] >> 5]) : 0u;
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u)
+                if ((vis[u] >> (row[u] & 31)) & 1u) live &= ~(1u << u);
+        }
+        if (LAZY) {
+#pragma unroll
+            for (uint32_t u = 0; u < 4; ++u)
+                if ((live >> u) & 1u) atomicOr(&fcur[row[u] >> 5], 1u << (row[u] & 31));
+            continue;
+        }
+        // the claims and the winners' list bounds in flight together
+        uint32_t old[4], b[4], d[4], won = 0;
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u)
+            old[u] = (live >> u) & 1u ? atomicOr(&a.visited[row[u] >> 5], 1u << (row[u] & 31)) : 0xFFFFFFFFu;
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u) {
+            b[u] = (live >> u) & 1u ? __ldg(&g.out_ptrs[row[u]]) : 0u;
+            d[u] = (live >> u) & 1u ? __ldg(&g.out_ptrs[row[u] + 1]) : 0u;
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u) {
+            if ((old[u] >> (row[u] & 31)) & 1u) continue;
+            won |= 1u << u;
+            d[u] -= b[u];
+            a.levels[row[u]] = level;
+            if (PARENTS) a.parents[row[u]] = src[u];
+            ++disc;
+            deg += own_lists ? __ldg(&g.csr_ptrs[row[u] + 1]) - __ldg(&g.csr_ptrs[row[u]]) : d[u];
+        }
+        emit(a, B, row, b, d, won, tail);
+    }
+}
+
+// A push level over the frontier's entries in the global queues: batches of
+// short lists, spread over the warps, then each warp's share of the long
+// lists' pieces (its first piece's entry by a 32-way search).
+template <bool PARENTS, bool LAZY>
+__device__ __forceinline__ void push_level(const BfsArgs& a, BlockState& B, const Run& s, uint32_t warp,
+                                           uint32_t nwarps, bool precheck, uint32_t* fcur, const Tail& tail,
+                                           uint32_t& disc, uint32_t& deg) {
+    const uint32_t lane = threadIdx.x & 31;
+    {
+        const uint4* q = a.pieces + s.from.a;
+        const uint32_t T = s.size.a, per = min(32u, (T + nwarps - 1) / nwarps);
+        for (uint64_t e0 = (uint64_t)warp * per; e0 < T; e0 += (uint64_t)nwarps * per) {
+            uint4 p = make_uint4(0u, 0u, 0u, 0u);
+            if (lane < per && e0 + lane < T) p = __ldcg(&q[e0 + lane]);
+            push_batch<PARENTS, LAZY>(a, B, p, s.level, precheck, fcur, tail, disc, deg);
+        }
+    }
+    const uint4* q = a.pieces + a.g.n + s.from.b;
+    const uint32_t T = s.size.b, U = s.size.u;
+    // with few pieces a warp takes one; shares start at the other end of the
+    // warps, which have no short lists
+    const uint32_t share = (U + nwarps - 1) / nwarps;
+    uint32_t x = (nwarps - 1 - warp) * share;
+    const uint32_t end = min(U, x + share);
+    if (x >= end) return;
+    uint32_t lo = 0, hi = T;
+    while (hi - lo > 32) {
+        const uint32_t step = (hi - lo + 31) / 32, idx = lo + lane * step;
+        const bool ok = idx < hi && __ldcg(&q[idx].w) <= x;
+        const uint32_t nlo = lo + (__popc(__ballot_sync(0xFFFFFFFFu, ok)) - 1) * step;
+        hi = min(hi, nlo + step);
+        lo = nlo;
+    }
+    {
+        const bool ok = lo + lane < hi && __ldcg(&q[lo + lane].w) <= x;
+        lo += __popc(__ballot_sync(0xFFFFFFFFu, ok)) - 1;
+    }
+    while (x < end) {
+        // lane j takes piece x + j, while it lies in the share
+        const uint32_t take = min(32u, end - x);
+        // entries lo .. lo + 31 cover at least 32 pieces from x on
+        const uint4 e = lo + lane < T ? __ldcg(&q[lo + lane]) : make_uint4(0u, 0u, 0u, 0xFFFFFFFFu);
+        uint32_t own = 0;
+#pragma unroll
+        for (uint32_t st = 16; st > 0; st >>= 1) {
+            const uint32_t o = __shfl_sync(0xFFFFFFFFu, e.w, own + st);
+            if (o <= x + lane) own += st;
+        }
+        const uint32_t eb = __shfl_sync(0xFFFFFFFFu, e.x, own), ed = __shfl_sync(0xFFFFFFFFu, e.y, own);
+        const uint32_t ev = __shfl_sync(0xFFFFFFFFu, e.z, own), ew = __shfl_sync(0xFFFFFFFFu, e.w, own);
+        uint4 p = make_uint4(0u, 0u, 0u, 0u);
+        if (lane < take) {
+            const uint32_t k = (x + lane - ew) * kPiece;
+            if (k < ed) p = make_uint4(eb + k, min(kPiece, ed - k), ev, 0u);
+            else set_error(a.ctr, BLEST_ERR_DEVICE_INDEX);  // offsets and lengths disagree: cannot happen
+        }
+        push_batch<PARENTS, LAZY>(a, B, p, s.level, precheck, fcur, tail, disc, deg);
+        x += take;
+        lo += __shfl_sync(0xFFFFFFFFu, own, take - 1);
+    }
+}
+
+// End of a level (or of a part of it): the grid barrier, then thread 0 reads
+// the level's counters. Adds the block's disc/deg first when `add`. Returns
+// false when the run has an error recorded.
+__device__ __forceinline__ bool level_end(const BfsArgs& a, BlockState& B, unsigned long long* lvl, bool add,
+                                          uint32_t disc, uint32_t deg) {
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    if (add) {
+        disc = __reduce_add_sync(0xFFFFFFFFu, disc);
+        deg = __reduce_add_sync(0xFFFFFFFFu, deg);
+        if (lane == 0) {
+            B.tot_disc[w] = disc;
+            B.tot_deg[w] = deg;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (add) {
+            uint32_t sd = 0, sg = 0;
+            for (uint32_t i = 0; i < nw; ++i) {
+                sd += B.tot_disc[i];
+                sg += B.tot_deg[i];
+            }
+            if (sd) {
+                atomicAdd(&lvl[1], (unsigned long long)sd);
+                atomicAdd(&lvl[2], (unsigned long long)sg);
+            }
+        }
+        const uint64_t v = barrier_arrive_wait(a.ctr);
+#pragma unroll
+        for (uint32_t i = 0; i < kSlotWords; ++i) B.val[i] = ld_relaxed64(&lvl[i]);
+        B.ok = (v & kArriveError) == 0;
+    }
+    __syncthreads();
+    return B.ok;
+}
+
+__device__ __forceinline__ void trace_level(const BfsArgs& a, uint32_t level, int dir, uint32_t nf, uint32_t units) {
+    if (!a.trace || level > BLEST_TRACE_CAPACITY) return;
+    blest_level_trace& t = a.trace[level - 1];
+    t.start_ns = global_ns();
+    t.level = level;
+    t.direction = (uint32_t)dir;
+    t.frontier = nf;
+    t.work_units = units;
+    t.sweep_ns = 0;
+    t.longest_scan = 0;
+}
+
+// Levels run by block 0 alone, from the queues on, until the frontier outgrows
+// a block (its entries are then in the global queues again), is empty, or
+// kSoloLevels are done.
+template <bool PARENTS>
+__device__ __forceinline__ void solo_levels(const BfsArgs& a, BlockState& B, Run& s, const Tail& tail) {
+    RunCounters* c = a.ctr;
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    uint32_t T = s.size.a + s.size.u, done = 0;
+    for (uint32_t i = threadIdx.x; i < s.size.a; i += blockDim.x) B.solo[i] = __ldcg(&a.pieces[s.from.a + i]);
+    for (uint32_t i = threadIdx.x; i < s.size.b; i += blockDim.x) {
+        const uint4 e = __ldcg(&a.pieces[a.g.n + s.from.b + i]);
+        for (uint32_t k = 0; k < e.y; k += kPiece)
+            B.solo[s.size.a + e.w + k / kPiece] = make_uint4(e.x + k, min(kPiece, e.y - k), e.z, 0u);
+    }
+    __syncthreads();
+    for (bool inside = true; inside;) {
+        const uint32_t nf = s.D1 - s.D2;
+        if (threadIdx.x == 0) {
+            ++c->push_levels;
+            if (done) trace_level(a, s.level, BLEST_DIR_PUSH, nf, T);
+        }
+        s.nf_prev = nf;
+        uint32_t disc = 0, deg = 0;
+        const uint32_t per = min(32u, (T + nw - 1) / nw);
+        for (uint32_t e0 = w * per; e0 < T; e0 += nw * per) {
+            uint4 p = make_uint4(0u, 0u, 0u, 0u);
+            if (lane < per && e0 + lane < T) p = B.solo[e0 + lane];
+            push_batch<PARENTS, false>(a, B, p, s.level, false, nullptr, tail, disc, deg);
+        }
+        ++done;
+        const Flushed F = flush(a, B, tail, nullptr, disc, deg, done < kSoloLevels);
+        s.D2 = s.D1;
+        s.G2 = s.G1;
+        s.D1 += F.disc;
+        s.G1 += F.deg;
+        ++s.level;
+        T = F.pieces;
+        inside = F.in_solo && F.disc && s.level <= a.g.n + 1;
+        __syncthreads();  // B.solo and the buffer's reset are visible
+    }
+    if (threadIdx.x == 0) {
+        // what the last level left in the global queues; two records in turn:
+        // a block may still be reading the last one (degree sums are below
+        // 2^32, as nnz is)
+        s.from.a += s.size.a;
+        s.from.b += s.size.b;
+        s.size = span_of(ld_relaxed64(tail.ca), ld_relaxed64(tail.cb));
+        unsigned long long* r = c->solo[s.step % 2];
+        r[0] = ((unsigned long long)s.nf_prev << 32) | s.level;
+        r[1] = ((unsigned long long)s.from.a << 32) | s.size.a;
+        r[2] = ((unsigned long long)s.from.b << 32) | s.size.b;
+        r[3] = s.size.u;
+        r[4] = ((unsigned long long)s.D2 << 32) | s.D1;
+        r[5] = (s.G2 << 32) | s.G1;
+    }
+}
+
+// Bottom-up level: a warp owns the words wi = warp + t * nwarps and takes them
+// 32 at a time: lane j loads word j's visited and has-in words, and the
+// unvisited vertices with in-neighbours of all 32 words are compacted into
+// one list (a warp scan of their counts) that the lanes take 32 at a time, so
+// no lane idles on a visited vertex. Each lane scans its vertex's
+// in-neighbours four at a time (independent loads) for at most kPullLaneScan
+// neighbours; the warp then finishes the longer lists together, 32 neighbours
+// per coalesced step, stopping at the first frontier neighbour; very long
+// lists go to the heavy queue. The next round's row bounds are loaded while
+// the current round is scanned. Found vertices set their bit in the warp's
+// word slots in shared memory; after the chunk lane j writes word j's visited
+// and frontier words. A
+// neighbour's frontier word is read, through L1 (nobody writes it in this
+// level), only when the summary in shared memory says it is non-empty.
+template <bool PARENTS, class InFrontier>
+__device__ __forceinline__ void pull_level(const BfsArgs& a, BlockState& B, uint32_t level, uint32_t warp,
+                                           uint32_t nwarps, uint32_t* fcur, uint32_t* fsum, unsigned long long* lvl,
+                                           InFrontier in_frontier, uint32_t& disc, uint32_t& deg) {
+    const uint32_t lane = threadIdx.x & 31;
+    const DevGraph& g = a.g;
+    const uint32_t W = (g.n + 31) / 32;
+    const uint32_t tailMask = (g.n & 31) ? ((1u << (g.n & 31)) - 1) : 0xFFFFFFFFu;
+    uint32_t longest = 0;
+    uint32_t* found_slots = B.found + (threadIdx.x & ~31u);
+    for (uint32_t t0 = 0; warp + t0 * nwarps < W; t0 += 32) {
+        const uint32_t wj = warp + (t0 + lane) * nwarps;
+        uint32_t visj = 0xFFFFFFFFu, unvj = 0;
+        if (wj < W) {
+            visj = __ldcg(&a.visited[wj]);
+            const uint32_t hj = g.has_in ? __ldg(&g.has_in[wj]) : 0xFFFFFFFFu;
+            unvj = ~visj & hj & (wj == W - 1 ? tailMask : 0xFFFFFFFFu);
+        }
+        // exclusive offsets of the words' items in the chunk's list
+        const uint32_t cj = __popc(unvj);
+        uint32_t incl = cj;
+#pragma unroll
+        for (uint32_t d = 1; d < 32; d <<= 1) {
+            const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+            if (lane >= d) incl += o;
+        }
+        const uint32_t offj = incl - cj;
+        const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+        if (total == 0) continue;
+        found_slots[lane] = 0u;
+        __syncwarp();
+        // item idx -> (word slot, vertex); warp-uniform call
+        auto item = [&](uint32_t idx, uint32_t& slot, uint32_t& vtx) {
+            uint32_t lo = 0;
+#pragma unroll
+            for (uint32_t st = 16; st > 0; st >>= 1) {
+                const uint32_t o = __shfl_sync(0xFFFFFFFFu, offj, lo + st);
+                if (o <= idx) lo += st;
+            }
+            const uint32_t o = __shfl_sync(0xFFFFFFFFu, offj, lo);
+            const uint32_t um = __shfl_sync(0xFFFFFFFFu, unvj, lo);
+            slot = lo;
+            vtx = idx < total ? (warp + (t0 + lo) * nwarps) * 32 + __fns(um, 0, (int)(idx - o + 1)) : kUnreached;
+        };
+        uint32_t nslot, nvtx;
+        item(lane, nslot, nvtx);
+        uint32_t npb = nvtx < g.n ? __ldg(&g.csr_ptrs[nvtx]) : 0u;
+        uint32_t npe = nvtx < g.n ? __ldg(&g.csr_ptrs[nvtx + 1]) : 0u;
+        for (uint32_t base = 0; base < total; base += 32) {
+            const uint32_t myslot = nslot, u = nvtx, pb = npb, pe = npe;
+            if (base + 32 < total) {
+                item(base + 32 + lane, nslot, nvtx);
+                npb = nvtx < g.n ? __ldg(&g.csr_ptrs[nvtx]) : 0u;
+                npe = nvtx < g.n ? __ldg(&g.csr_ptrs[nvtx + 1]) : 0u;
+            }
+            bool found = false;
+            uint32_t parent = kUnreached, p = pb;
+            if (u < g.n) {
+                const uint32_t cap = pb + min(pe - pb, kPullLaneScan);
+                for (; p < cap && !found; p += kPullUnroll) {
+                    uint32_t v[kPullUnroll];
+                    bool f[kPullUnroll];
+#pragma unroll
+                    for (uint32_t j = 0; j < kPullUnroll; ++j)
+                        v[j] = p + j < pe ? __ldg(&g.csr_ids[p + j]) : kUnreached;
+#pragma unroll
+                    for (uint32_t j = 0; j < kPullUnroll; ++j) f[j] = v[j] != kUnreached && in_frontier(v[j]);
+#pragma unroll
+                    for (uint32_t j = 0; j < kPullUnroll; ++j) {
+                        if (!found && f[j]) {
+                            found = true;
+                            parent = v[j];
+                        }
+                    }
+                }
+            }
+            // Very long lists go to the heavy queue (all warps split them
+            // after the level barrier).
+            if (!found && p < pe && pe - p > a.heavy_min) {
+                const uint32_t chunks = (pe - p + kHeavyChunk - 1) / kHeavyChunk;
+                const uint64_t hs = atomicAdd(&lvl[3], (unsigned long long)((1ull << kQShift) | chunks));
+                const uint32_t idx = (uint32_t)(hs >> kQShift);
+                if (idx < a.heavy_cap) {
+                    a.heavy[idx] = make_uint4(u, p, pe, (uint32_t)(hs & kQUnitMask));
+                    p = pe;  // handed over
+                } else {
+                    set_error(a.ctr, BLEST_ERR_DEVICE_INDEX);  // capacity is sized so this cannot happen
+                }
+            }
+            // Long lists: the whole warp scans them, one vertex at a time.
+            for (uint32_t rest = __ballot_sync(0xFFFFFFFFu, !found && p < pe); rest; rest &= rest - 1) {
+                const uint32_t ln = __ffs(rest) - 1;
+                const uint32_t q0 = __shfl_sync(0xFFFFFFFFu, p, ln);
+                const uint32_t q1 = __shfl_sync(0xFFFFFFFFu, pe, ln);
+                longest = max(longest, q1 - q0);
+                uint32_t hitv = kUnreached;
+                for (uint32_t qb = q0; qb < q1; qb += 32) {
+                    const uint32_t idx = qb + lane;
+                    const uint32_t v = idx < q1 ? __ldg(&g.csr_ids[idx]) : kUnreached;
+                    const uint32_t hb = __ballot_sync(0xFFFFFFFFu, v != kUnreached && in_frontier(v));
+                    if (hb) {
+                        hitv = __shfl_sync(0xFFFFFFFFu, v, __ffs(hb) - 1);
+                        break;
+                    }
+                }
+                if (lane == ln && hitv != kUnreached) {
+                    found = true;
+                    parent = hitv;
+                }
+            }
+            if (found) {
+                a.levels[u] = level;
+                if (PARENTS) a.parents[u] = parent;
+                ++disc;
+                deg += pe - pb;
+            }
+            // this round's found bits, merged per word slot by a warp
+            // reduction: one store per distinct slot (lanes of one word
+            // would otherwise collide on the same shared-memory word)
+            for (uint32_t pending = __ballot_sync(0xFFFFFFFFu, found); pending;) {
+                const uint32_t slot = __shfl_sync(0xFFFFFFFFu, myslot, __ffs(pending) - 1);
+                const bool mine = found && myslot == slot;
+                const uint32_t bits = __reduce_or_sync(0xFFFFFFFFu, mine ? 1u << (u & 31) : 0u);
+                if (lane == 0) found_slots[slot] |= bits;
+                pending &= ~__ballot_sync(0xFFFFFFFFu, mine);
+            }
+        }
+        __syncwarp();
+        // write back the chunk's words (lane j: word j)
+        const uint32_t nb = found_slots[lane];
+        __syncwarp();
+        if (nb) {
+            fcur[wj] = nb;
+            a.visited[wj] = visj | nb;
+            mark_summary(a, fsum, wj);
+        }
+    }
+    if (a.trace && lane == 0 && longest && level <= BLEST_TRACE_CAPACITY)
+        atomicMax((unsigned long long*)&a.trace[level - 1].longest_scan, (unsigned long long)longest);
+}
+
+// The heavy lists of a pull level: every warp takes an equal share of their
+// pieces.
+template <bool PARENTS, class InFrontier>
+__device__ __forceinline__ void heavy_level(const BfsArgs& a, uint64_t hq, uint32_t level, uint32_t warp,
+                                            uint32_t nwarps, uint32_t* fcur, uint32_t* fsum, InFrontier in_frontier,
+                                            uint32_t& disc, uint32_t& deg) {
+    const uint32_t lane = threadIdx.x & 31;
+    const DevGraph& g = a.g;
+    const uint32_t hitems = min((uint32_t)(hq >> kQShift), a.heavy_cap);
+    const uint32_t hchunks = (uint32_t)(hq & kQUnitMask);
+    const uint32_t hk = (hchunks + nwarps - 1) / nwarps;
+    for (uint32_t ch = warp * hk; hitems && ch < min(hchunks, warp * hk + hk); ++ch) {
+        // owner: largest item with chunk offset <= ch
+        uint32_t lo = 0, hi = hitems;
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) / 2;
+            if (__ldcg(&a.heavy[mid].w) <= ch) lo = mid;
+            else hi = mid;
+        }
+        const uint4 it = __ldcg(&a.heavy[lo]);
+        const uint32_t hu = it.x, w = hu >> 5, b = 1u << (hu & 31);
+        const uint32_t q0 = it.y + (ch - it.w) * kHeavyChunk;
+        const uint32_t q1 = min(it.z, q0 + kHeavyChunk);
+        uint32_t hitv = kUnreached;
+        for (uint32_t base = q0; base < q1 && hitv == kUnreached; base += 32) {
+            if (__ldcg(&a.visited[w]) & b) break;  // another piece found it
+            const uint32_t idx = base + lane;
+            const uint32_t v = idx < q1 ? __ldg(&g.csr_ids[idx]) : kUnreached;
+            const uint32_t hb = __ballot_sync(0xFFFFFFFFu, v != kUnreached && in_frontier(v));
+            if (hb) hitv = __shfl_sync(0xFFFFFFFFu, v, __ffs(hb) - 1);
+        }
+        if (hitv != kUnreached && lane == 0 && !(atomicOr(&a.visited[w], b) & b)) {
+            a.levels[hu] = level;
+            if (PARENTS) a.parents[hu] = hitv;
+            ++disc;
+            deg += __ldg(&g.csr_ptrs[hu + 1]) - __ldg(&g.csr_ptrs[hu]);
+            atomicOr(&fcur[w], b);
+            mark_summary(a, fsum, w);
+        }
+    }
+}
+
+template <bool PARENTS>
+__device__ __forceinline__ void lists_run(const BfsArgs& a) {
+    extern __shared__ uint32_t s_sum[];
+    __shared__ BlockState B;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t nth = gridDim.x * blockDim.x;
+    // warps are numbered across the blocks, so that a few busy ones lie on
+    // different SMs
+    const uint32_t warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    const uint32_t nwarps = nth >> 5;
+    const DevGraph& g = a.g;
+    const uint32_t n = g.n;
+    RunCounters* c = a.ctr;
+
+    // ---- level 0: outputs and bitmaps reset, the source's pieces queued (the
+    // run counters were zeroed by the launcher)
+    Run s{};
+    {
+        const uint32_t src = a.src;
+        for (uint32_t v = tid; v < n; v += nth) {
+            a.levels[v] = v == src ? 0u : kUnreached;
+            if (PARENTS) a.parents[v] = v == src ? src : kUnreached;
+        }
+        const uint32_t sw = src >> 5, sb = 1u << (src & 31);
+        for (uint32_t i = tid; i < a.words; i += nth) {
+            a.visited[i] = i == sw ? sb : 0u;
+            a.frontier0[i] = 0u;
+            a.frontier1[i] = 0u;
+            a.frontier2[i] = 0u;
+        }
+        for (uint32_t i = tid; i < a.sum_words; i += nth) {
+            a.summary0[i] = 0u;
+            a.summary1[i] = 0u;
+            a.summary2[i] = 0u;
+        }
+        const uint32_t b = __ldg(&g.out_ptrs[src]), d = __ldg(&g.out_ptrs[src + 1]) - b;
+        s.level = 1;
+        if (tid == 0) {
+            Span at{0u, 0u, 0u};
+            put_entry(a, at, src, b, d);
+        }
+        s.size = d > kPiece ? Span{0u, 1u, pieces_of(d)} : Span{d ? 1u : 0u, 0u, 0u};
+        s.D1 = 1;
+        s.G1 = __ldg(&g.csr_ptrs[src + 1]) - __ldg(&g.csr_ptrs[src]);
+        if (threadIdx.x == 0) {
+            B.win_cnt = 0;
+            B.win_end = kWinners;
+        }
+    }
+    if (!grid_barrier(c)) return;
+
+    int dir = a.direction == BLEST_DIR_PULL ? BLEST_DIR_PULL : BLEST_DIR_PUSH;
+    bool queued = true;  // the frontier is in the queue (else: bitmap `gen`)
+    uint32_t gen = 0;    // bitmaps made; bitmap gen + 1 is zero (its clearing is part of making gen)
+    const uint32_t W = (n + 31) / 32;
+    auto clear_next = [&]() {
+        uint32_t* f = bitmap_of(a, gen + 1);
+        uint32_t* m = summary_of(a, gen + 1);
+        for (uint32_t i = tid; i < a.words; i += nth) f[i] = 0u;
+        for (uint32_t i = tid; i < a.sum_words; i += nth) m[i] = 0u;
+    };
+
+    for (;;) {
+        const uint32_t level = s.level;
+        const uint32_t nf = s.D1 - s.D2;  // discovered at level - 1
+        const uint64_t mf = s.G1 - s.G2;  // their edges
+        if (nf == 0 || level > n + 1) {
+            if (tid == 0) {
+                c->discovered = s.D1;
+                c->degree = s.G1;
+                if (nf == 0) {
+                    c->levels = level - 1;  // max level + 1
+                    trace_level(a, level, 0, 0, 0);
+                }
+            }
+            if (nf != 0) set_error(c, BLEST_ERR_LEVEL_CAP);
+            break;
+        }
+        if (a.direction == BLEST_DIR_AUTO) {
+            // Beamer's switch in edge/vertex units: to pull when the new
+            // frontier's edges m_f exceed the unvisited edges m_u / alpha and
+            // the frontier grows; back to push when it has fewer than n / beta
+            // vertices. Going to pull also needs m_f above 8 edges per
+            // bitmap word, going back below that: a pull level visits every
+            // word, so a grid's growing wavefront (4.6 edges a word at its
+            // widest, which passes Beamer's test) is better off pushing.
+            const double bar = 8.0 * (double)W;
+            if (dir == BLEST_DIR_PUSH) {
+                if ((double)mf * a.alpha > (double)(g.degree_total - s.G1) && nf > s.nf_prev && (double)mf > bar)
+                    dir = BLEST_DIR_PULL;
+            } else if ((double)nf * a.beta < (double)n && (double)mf < bar) {
+                dir = BLEST_DIR_PUSH;
+            }
+        }
+        if (tid == 0) trace_level(a, level, dir, nf, queued ? s.size.a + s.size.u : nf);
+        unsigned long long* lvl = c->lvl[s.step % 3];
+        // the next step's counters (their slot was last read two steps back)
+        if (tid < kSlotWords) c->lvl[(s.step + 1) % 3][tid] = 0;
+        // the queues end where the frontier's entries end
+        const Span next{s.from.a + s.size.a, s.from.b + s.size.b, 0u};
+        uint32_t disc = 0, deg = 0;
+
+        // ---- the frontier in the form this direction reads
+        if (dir == BLEST_DIR_PUSH && !queued) {
+            const Tail tail{next, &lvl[3], &lvl[5]};
+            const uint32_t* f = bitmap_of(a, gen);
+            for (uint32_t base = warp * 32; base < W; base += nwarps * 32) {
+                uint32_t bits = base + lane < W ? __ldcg(&f[base + lane]) : 0u;
+                while (__any_sync(0xFFFFFFFFu, bits)) {
+                    uint32_t v[4], b[4], d[4], won = 0;
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; ++k) {
+                        v[k] = b[k] = d[k] = 0u;
+                        if (bits) {
+                            v[k] = (base + lane) * 32 + __ffs(bits) - 1;
+                            bits &= bits - 1;
+                            won |= 1u << k;
+                            b[k] = __ldg(&g.out_ptrs[v[k]]);
+                            d[k] = __ldg(&g.out_ptrs[v[k] + 1]) - b[k];
+                        }
+                    }
+                    emit(a, B, v, b, d, won, tail);
+                }
+            }
+            flush(a, B, tail, nullptr, 0, 0, false);
+            if (!level_end(a, B, lvl, false, 0, 0)) return;
+            s.from = next;
+            s.size = span_of(B.val[3], B.val[5]);
+            queued = true;
+        } else if (dir == BLEST_DIR_PULL && queued) {
+            ++gen;
+            clear_next();
+            uint32_t* f = bitmap_of(a, gen);
+            uint32_t* m = summary_of(a, gen);
+            // a vertex without out-edges has no entry, and is nobody's in-neighbour
+            for (uint32_t e = tid; e < s.size.a + s.size.b; e += nth) {
+                const uint32_t at = e < s.size.a ? s.from.a + e : n + s.from.b + (e - s.size.a);
+                const uint32_t v = __ldcg(&a.pieces[at].z);
+                atomicOr(&f[v >> 5], 1u << (v & 31));
+                // many vertices share a summary word: look before the atomic
+                const uint32_t sb = (v >> 5) >> a.sum_shift;
+                if (!((__ldcg(&m[sb >> 5]) >> (sb & 31)) & 1u)) atomicOr(&m[sb >> 5], 1u << (sb & 31));
+            }
+            if (!grid_barrier(c)) return;
+            queued = false;
+        }
+
+        if (dir == BLEST_DIR_PUSH) {
+            const Span end{s.from.a + s.size.a, s.from.b + s.size.b, 0u};
+            const Tail tail{end, &lvl[0], &lvl[4]};
+            if (s.size.a + s.size.u <= kSoloPieces && mf <= kSoloEdges) {
+                if (blockIdx.x == 0) solo_levels<PARENTS>(a, B, s, tail);
+                if (!level_end(a, B, c->solo[s.step % 2], false, 0, 0)) return;
+                s.level = (uint32_t)B.val[0];
+                s.nf_prev = (uint32_t)(B.val[0] >> 32);
+                s.from = Span{(uint32_t)(B.val[1] >> 32), (uint32_t)(B.val[2] >> 32), 0u};
+                s.size = Span{(uint32_t)B.val[1], (uint32_t)B.val[2], (uint32_t)B.val[3]};
+                s.D1 = (uint32_t)B.val[4];
+                s.D2 = (uint32_t)(B.val[4] >> 32);
+                s.G1 = (uint32_t)B.val[5];
+                s.G2 = B.val[5] >> 32;
+                ++s.step;
+                continue;
+            }
+            // a large level looks before it claims: most ends are visited
+            const bool precheck = mf > 16384;
+            // Lazy level: when the frontier's edges exceed n / 4 the level
+            // discovers a large part of the graph; then an edge only marks its
+            // end (an atomic nobody waits for) and a word sweep keeps the
+            // unvisited ones and writes their levels, coalesced. While under
+            // an eighth of the graph is visited the look first would filter
+            // little.
+            if (!PARENTS && mf > (uint64_t)(n / 4)) {
+                ++gen;
+                clear_next();
+                uint32_t* fcur = bitmap_of(a, gen);
+                uint32_t* fsum = summary_of(a, gen);
+                push_level<PARENTS, true>(a, B, s, warp, nwarps, s.D1 > n / 8, fcur, tail, disc, deg);
+                if (!grid_barrier(c)) return;
+                if (a.trace && tid == 0 && level <= BLEST_TRACE_CAPACITY) a.trace[level - 1].sweep_ns = global_ns();
+                for (uint32_t base = warp * 32; base < W; base += nwarps * 32) {
+                    const uint32_t wi = base + lane;
+                    uint32_t nw = 0;
+                    if (wi < W) {
+                        const uint32_t cand = __ldcg(&fcur[wi]);
+                        if (cand) {
+                            const uint32_t vis = __ldcg(&a.visited[wi]);
+                            nw = cand & ~vis;
+                            fcur[wi] = nw;
+                            if (nw) {
+                                a.visited[wi] = vis | nw;
+                                mark_summary(a, fsum, wi);
+                            }
+                        }
+                    }
+                    // 8 words at a time, a lane per vertex: all their degree
+                    // loads are issued before any is added
+                    const uint32_t words = __ballot_sync(0xFFFFFFFFu, nw != 0);
+                    for (uint32_t j0 = 0; j0 < 32; j0 += 8) {
+                        if (!((words >> j0) & 0xFFu)) continue;
+                        uint32_t d0[8], d1[8], vb = 0;
+#pragma unroll
+                        for (uint32_t k = 0; k < 8; ++k) {
+                            const uint32_t bits = __shfl_sync(0xFFFFFFFFu, nw, j0 + k);
+                            const uint32_t v = (base + j0 + k) * 32 + lane;
+                            d0[k] = d1[k] = 0u;
+                            if ((bits >> lane) & 1u) {
+                                vb |= 1u << k;
+                                d0[k] = __ldg(&g.csr_ptrs[v]);
+                                d1[k] = __ldg(&g.csr_ptrs[v + 1]);
+                            }
+                        }
+#pragma unroll
+                        for (uint32_t k = 0; k < 8; ++k) {
+                            if ((vb >> k) & 1u) {
+                                a.levels[(base + j0 + k) * 32 + lane] = level;
+                                ++disc;
+                                deg += d1[k] - d0[k];
+                            }
+                        }
+                    }
+                }
+                queued = false;
+                if (tid == 0) c->push_levels++;
+                if (!level_end(a, B, lvl, true, disc, deg)) return;
+            } else {
+                push_level<PARENTS, false>(a, B, s, warp, nwarps, precheck, nullptr, tail, disc, deg);
+                flush(a, B, tail, lvl, disc, deg, false);
+                if (tid == 0) c->push_levels++;
+                if (!level_end(a, B, lvl, false, 0, 0)) return;
+                s.from = end;
+                s.size = span_of(B.val[0], B.val[4]);
+            }
+        } else {
+            const uint32_t* fprev = bitmap_of(a, gen);
+            const uint32_t* sprev = summary_of(a, gen);
+            for (uint32_t i = threadIdx.x; i < a.sum_words; i += blockDim.x) s_sum[i] = __ldcg(&sprev[i]);
+            ++gen;
+            clear_next();
+            uint32_t* fcur = bitmap_of(a, gen);
+            uint32_t* fsum = summary_of(a, gen);
+            auto in_frontier = [&](uint32_t v) -> bool {
+                const uint32_t sb = (v >> 5) >> a.sum_shift;
+                if (!((s_sum[sb >> 5] >> (sb & 31)) & 1u)) return false;
+                return (fprev[v >> 5] >> (v & 31)) & 1u;
+            };
+            __syncthreads();
+            pull_level<PARENTS>(a, B, level, warp, nwarps, fcur, fsum, lvl, in_frontier, disc, deg);
+            if (tid == 0) c->pull_levels++;
+            if (!level_end(a, B, lvl, true, disc, deg)) return;
+            if (B.val[3]) {
+                const uint64_t hq = B.val[3];
+                disc = deg = 0;
+                heavy_level<PARENTS>(a, hq, level, warp, nwarps, fcur, fsum, in_frontier, disc, deg);
+                if (!level_end(a, B, lvl, true, disc, deg)) return;
+            }
+        }
+        s.nf_prev = nf;
+        s.D2 = s.D1;
+        s.G2 = s.G1;
+        s.D1 += (uint32_t)B.val[1];
+        s.G1 += B.val[2];
+        ++s.level;
+        ++s.step;
+    }
+}
+
+template <bool PARENTS>
+__global__ void __launch_bounds__(512, 2) bfs_lists_kernel(BfsArgs a) {
+    const uint64_t t0 = global_ns();
+    lists_run<PARENTS>(a);
+    write_record(a, t0);
+}
+
+}  // namespace
+}  // namespace dev
+
+namespace {
+
+template <bool PARENTS>
+void launch_lists(const blest_graph* g, const dev::BfsArgs& args, int blocks_per_sm, int threads, uint32_t grid_cap,
+                  cudaStream_t s) {
+    auto kern = dev::bfs_lists_kernel<PARENTS>;
+    const size_t smem = 4ull * args.sum_words;
+    // Per (device, block size, shared memory): the attribute is set once
+    // (always the maximum, so concurrent calls for graphs of different sizes
+    // agree) and the occupancy is asked once; both are fixed per device.
+    static std::mutex mu;
+    static std::map<std::tuple<int, int, size_t>, int> occupancy;
+    int maxBlocks = 0;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        const auto key = std::make_tuple(g->device, threads, smem);
+        const auto it = occupancy.find(key);
+        if (it != occupancy.end()) {
+            maxBlocks = it->second;
+        } else {
+            BLEST_CUDA(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)kSummaryMaxBytes));
+            BLEST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxBlocks, kern, threads, smem));
+            occupancy[key] = maxBlocks;
+        }
+    }
+    if (maxBlocks < 1) throw Error(BLEST_ERR_CUDA, "BFS kernel cannot be resident with this block size");
+    const int bps = blocks_per_sm > 0 ? std::min(blocks_per_sm, maxBlocks) : maxBlocks;
+    // A small graph takes no more blocks than it has work for (2048 edges or
+    // 512 vertices each): every block costs every barrier.
+    const uint64_t work = std::max<uint64_t>(g->d.n / 512, g->d.nnz / 2048) + 1;
+    const int grid = (int)std::min<uint64_t>(cooperative_grid(bps, g->sm_count, grid_cap), work);
+    BLEST_CUDA(cudaMemsetAsync(args.ctr, 0, sizeof(dev::RunCounters), s));
+    void* kargs[] = {(void*)&args};
+    BLEST_CUDA(cudaLaunchCooperativeKernel((void*)kern, grid, threads, kargs, smem, s));
+}
+
+}  // namespace
+
+void launch_bfs_lists(const blest_graph* g, const dev::BfsArgs& args, int blocks_per_sm, int threads,
+                      uint32_t grid_cap, cudaStream_t s) {
+    if (args.parents) launch_lists<true>(g, args, blocks_per_sm, threads, grid_cap, s);
+    else launch_lists<false>(g, args, blocks_per_sm, threads, grid_cap, s);
+}
+
+}  // namespace blest

@@ -341,6 +341,60 @@ __global__ void tiles_symmetric_kernel(DevGraph g, uint32_t* seen, uint32_t* bad
     if (lane == 0 && count) atomicAdd(edges, (unsigned long long)count);
 }
 
+// Out-edges of every column (one warp per rset, which owns its 8 columns).
+__global__ void out_count_kernel(DevGraph g, uint32_t* degree, unsigned long long* edges) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+    uint64_t sum = 0;
+    for (uint32_t r = warp; r < g.no_real; r += nwarps) {
+        const uint32_t t1 = __ldg(&g.rset_tile[r + 1]);
+        uint32_t cnt[8] = {};
+        for (uint32_t t = __ldg(&g.rset_tile[r]) + lane; t < t1; t += 32) {
+            const uint32_t mask = __ldg(&g.masks[t]);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) cnt[j] += __popc(mask & (0x01010101u << j));
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t d = __reduce_add_sync(0xFFFFFFFFu, cnt[j]);
+            const uint32_t c = r * 8 + j;
+            if (lane == 0 && c < g.n) {
+                degree[c] = d;
+                sum += d;
+            }
+        }
+    }
+    if (lane == 0 && sum) atomicAdd(edges, (unsigned long long)sum);
+}
+
+// Out-lists: column j of a rset takes the rows of its slices in tile order.
+__global__ void out_fill_kernel(DevGraph g, const uint32_t* ptrs, uint32_t* ids) {
+    const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1u;
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t r = warp; r < g.no_real; r += nwarps) {
+        const uint32_t t0 = __ldg(&g.rset_tile[r]), t1 = __ldg(&g.rset_tile[r + 1]);
+        uint32_t at[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) at[j] = r * 8 + j < g.n ? ptrs[r * 8 + j] : 0u;
+        for (uint32_t b = t0; b < t1; b += 32) {
+            const uint32_t t = b + lane;
+            const uint4 rows = t < t1 ? __ldg(&g.row4[t]) : make_uint4(0, 0, 0, 0);
+            const uint32_t mask = t < t1 ? __ldg(&g.masks[t]) : 0u;
+            const uint32_t rowk[4] = {rows.x, rows.y, rows.z, rows.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const bool on = (mask >> (8 * k + j)) & 1u;
+                    const uint32_t m = __ballot_sync(0xFFFFFFFFu, on);
+                    if (on) ids[at[j] + __popc(m & below)] = rowk[k];
+                    at[j] += __popc(m);
+                }
+            }
+        }
+    }
+}
+
 }  // namespace dev
 
 namespace {
@@ -500,6 +554,39 @@ bool tiles_symmetric_device(const dev::DevGraph& d, cudaStream_t s) {
     BLEST_CUDA(cudaMemcpyAsync(&h, out, sizeof(Out), cudaMemcpyDeviceToHost, s));
     BLEST_CUDA(cudaStreamSynchronize(s));
     return !h.bad && h.edges == d.nnz;
+}
+
+bool out_lists_device(const dev::DevGraph& d, cudaStream_t s, OutLists& out) {
+    int dev = 0, sms = 0;
+    BLEST_CUDA(cudaGetDevice(&dev));
+    BLEST_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    Scratch tmp;
+    uint32_t* degree = tmp.get<uint32_t>((size_t)d.n + 1);
+    unsigned long long* edges = tmp.get<unsigned long long>(1);
+    BLEST_CUDA(cudaMemsetAsync(degree, 0, 4 * ((size_t)d.n + 1), s));
+    BLEST_CUDA(cudaMemsetAsync(edges, 0, 8, s));
+    dev::out_count_kernel<<<sms * 8, 256, 0, s>>>(d, degree, edges);
+    BLEST_CUDA(cudaGetLastError());
+    unsigned long long total = 0;
+    BLEST_CUDA(cudaMemcpyAsync(&total, edges, 8, cudaMemcpyDeviceToHost, s));
+    BLEST_CUDA(cudaStreamSynchronize(s));
+    if (total >= 0xFFFFFF00ull) return false;
+    out = OutLists{};
+    out.edges = (uint32_t)total;
+    try {
+        out.ptrs = dmalloc<uint32_t>((size_t)d.n + 1);
+        out.ids = dmalloc<uint32_t>(total);
+        exclusive_scan(degree, out.ptrs, d.n + 1, s);
+        dev::out_fill_kernel<<<sms * 8, 256, 0, s>>>(d, out.ptrs, out.ids);
+        BLEST_CUDA(cudaGetLastError());
+        BLEST_CUDA(cudaStreamSynchronize(s));
+    } catch (...) {
+        cudaFree(out.ptrs);
+        cudaFree(out.ids);
+        out = OutLists{};
+        throw;
+    }
+    return true;
 }
 
 void device_bvss_free(DeviceBvss& b) {

@@ -43,7 +43,15 @@ struct DevGraph {
     // edges: {vertex, first edge, end edge, 0}, by vertex (multi-source pull).
     const uint4* pull_chunks;
     uint32_t no_pull_chunks;
+    // Out-neighbour lists (single-source push): those of the tiles' edges; the
+    // pull lists themselves when the graph is symmetric. Null: not kept.
+    const uint32_t* out_ptrs;  // n + 1
+    const uint32_t* out_ids;
+    uint32_t piece_cap;        // BFS queue entries: one per vertex, and one more per kBfsPieceEdges edges for long lists
 };
+
+// Most edges of one piece of the BFS push queue.
+constexpr uint32_t kBfsPieceEdges = 128;
 
 // Longest in-list one lane scans whole in the multi-source pull; longer
 // lists are scanned as pieces of this many edges.
@@ -51,6 +59,9 @@ constexpr uint32_t kPullChunk = 64;
 
 // Bit 63 of the barrier's arrival counter: some block recorded an error.
 constexpr unsigned long long kArriveError = 1ull << 63;
+
+// Words of one per-level counter slot.
+constexpr uint32_t kSlotWords = 6;
 
 // Counters of one BFS/CC/MBFS run (zeroed before every run).
 struct RunCounters {
@@ -66,11 +77,15 @@ struct RunCounters {
     // Slots reused across levels/iterations (queue counters, heavy-list
     // counters, trace maxima); each kernel documents its own use.
     unsigned long long aux[8];
-    // BFS per-level counters, slot = level % 3: packed queue entries/units
-    // added during the level, vertices discovered, their degree sum.
+    // BFS per-level counters, slot = level % 3 (step % 3 over lists): packed
+    // queue entries/units added during the level, vertices discovered, their
+    // degree sum, heavy in-lists; over lists also the short-list and long-list
+    // queue entries (words 0 and 4; 3 and 5 when a bitmap becomes a queue).
     // Counters of level L are read after the barrier that ends L and
     // zeroed during level L + 2, so no block ever needs a snapshot.
-    unsigned long long lvl[3][4];
+    unsigned long long lvl[3][kSlotWords];
+    // BFS over lists: where block 0 stood after running levels alone.
+    unsigned long long solo[2][kSlotWords];
     // Grid barrier: monotone arrival count (bits 0-62) + error flag (bit 63),
     // alone on its 128-byte line.
     alignas(128) unsigned long long arrive;

@@ -16,6 +16,10 @@
 
 namespace blest {
 
+namespace dev {
+struct BfsArgs;
+}
+
 void check_cuda(cudaError_t e, const char* what);
 #define BLEST_CUDA(x) ::blest::check_cuda((x), #x)
 
@@ -37,6 +41,7 @@ struct Workspace {
     uint32_t* summary[3] = {nullptr, nullptr, nullptr};  // frontier summaries
     uint32_t sum_shift = 0;                     // frontier words per summary bit = 2^sum_shift
     uint32_t sum_words = 0;                     // 32-bit words per summary
+    uint4* pieces = nullptr;                    // BFS push over lists: the queue
     uint4* heavy = nullptr;                     // pull: very long in-neighbour lists
     uint32_t heavy_cap = 0;
     uint32_t grid_blocks = 0;                   // cap on cooperative grid size (0 = whole GPU)
@@ -116,6 +121,8 @@ void workspace_free(Workspace& w);
 // w.records[seq % kRecordRing].
 void launch_bfs(const blest_graph* g, Workspace& w, uint32_t src, uint32_t* levels, uint32_t* parents,
                 const blest_bfs_params& p, cudaStream_t s, uint64_t seq);
+void launch_bfs_lists(const blest_graph* g, const dev::BfsArgs& args, int blocks_per_sm, int threads,
+                      uint32_t grid_cap, cudaStream_t s);
 void launch_cc(const blest_graph* g, Workspace& w, uint32_t* labels, cudaStream_t s);
 
 int device_sm_count(int device);
@@ -153,6 +160,14 @@ void compact_tiles_device(const uint32_t* row_ids, const uint32_t* masks, const 
 // sorted by descending list length, ties by id) hold exactly its edges, each
 // once. Blocking; every edge is looked up, nothing is sampled or hashed.
 bool tiles_symmetric_device(const dev::DevGraph& d, cudaStream_t s);
+// Out-neighbour lists of the tiles' edges, in device memory the caller owns.
+// False (and nothing allocated) when they are 2^32 or more.
+struct OutLists {
+    uint32_t* ptrs = nullptr;  // n + 1
+    uint32_t* ids = nullptr;
+    uint32_t edges = 0;
+};
+bool out_lists_device(const dev::DevGraph& d, cudaStream_t s, OutLists& out);
 void mbfs_scratch_free(void* p);
 // Allocate the multi-source BFS state of `words` 32-bit words per vertex now.
 void mbfs_reserve(Workspace& w, uint32_t n, uint32_t words);

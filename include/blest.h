@@ -239,10 +239,10 @@ int blest_workspace_set_grid(blest_workspace* ws, uint32_t blocks);
 
 /* ---- single-source BFS -------------------------------------------------- */
 #define BLEST_DIR_AUTO 0       /* direction-optimising (push <-> pull) */
-#define BLEST_DIR_PUSH 1       /* top-down over BVSS tiles only        */
+#define BLEST_DIR_PUSH 1       /* top-down only (out-lists; BVSS tiles with the MMA test) */
 #define BLEST_DIR_PULL 2       /* bottom-up over CSR only (after level 1) */
-#define BLEST_TEST_CUDA_CORE 0 /* slice test: (mask byte & frontier byte) != 0 */
-#define BLEST_TEST_B1_MMA 1    /* slice test: mma.sync m8n8k128 b1 AND+POPC (Common.cuh:57-66) */
+#define BLEST_TEST_CUDA_CORE 0 /* no slice test: push reads the frontier's out-lists */
+#define BLEST_TEST_B1_MMA 1    /* push over tiles, slice test: mma.sync m8n8k128 b1 AND+POPC (Common.cuh:57-66) */
 typedef struct blest_bfs_params {
     int direction;            /* BLEST_DIR_* */
     int slice_test;           /* BLEST_TEST_* */
@@ -261,7 +261,8 @@ typedef struct blest_level_trace {
     uint32_t level;
     uint32_t direction;       /* BLEST_DIR_PUSH or BLEST_DIR_PULL; 0 for the end record */
     uint64_t frontier;        /* vertices discovered at the previous level */
-    uint64_t work_units;      /* tiles (32-tile chunks with the MMA test) of the queued rsets */
+    uint64_t work_units;      /* push: pieces (<= 128 edges) of the frontier's out-lists (32-tile
+                                 chunks of the queued rsets with the MMA test); pull: frontier */
     uint64_t longest_scan;    /* pull: longest in-neighbour list finished by a whole warp */
     uint64_t sweep_ns;        /* lazy push level: %globaltimer when its word sweep started (0 otherwise) */
 } blest_level_trace;
