@@ -383,7 +383,10 @@ void graph_attach_csr(blest_graph* g, const blest_csr_view* csr, bool symmetric)
                 return dx != dy ? dx > dy : x < y;
             });
         }
-        d.csr_ids = blest::upload(g, ids.data(), ids.size());
+        // (room for whole 16-byte quads past the last list)
+        uint32_t* dids = blest::dev_alloc<uint32_t>(g, ids.size() + 8);
+        if (!ids.empty()) BLEST_CUDA(cudaMemcpy(dids, ids.data(), 4 * ids.size(), cudaMemcpyHostToDevice));
+        d.csr_ids = dids;
     }
     {
         std::vector<uint32_t> hasIn(((size_t)csr->n + 31) / 32 + 4, 0u);
@@ -415,6 +418,11 @@ void graph_attach_csr(blest_graph* g, const blest_csr_view* csr, bool symmetric)
         d.out_ptrs = out.ptrs;
         d.out_ids = out.ids;
         out_edges = out.edges;
+    }
+    if (d.out_ptrs) {
+        uint4* heads = blest::dev_alloc<uint4>(g, csr->n);
+        blest::list_heads_device(d, heads, nullptr);
+        d.heads = heads;
     }
     d.piece_cap = (uint32_t)(csr->n + out_edges / blest::dev::kBfsPieceEdges + 64);
     BLEST_CUDA(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));

@@ -49,6 +49,9 @@ namespace dev {
 namespace {
 
 constexpr uint32_t kPiece = kBfsPieceEdges;
+constexpr uint32_t kPullWords = 16;     // words a warp takes at a time in a pull level
+constexpr uint32_t kPullItems = 2;      // vertices a lane tries at a time
+constexpr uint32_t kPullWarpScan = 128; // list remainders above this are scanned by the whole warp
 constexpr uint32_t kMaxWarps = 16;      // per block (512 threads)
 constexpr uint32_t kWinners = 2048;     // discoveries a block gathers before it appends one warp at a time
 // A level is run by block 0 alone when its pieces and edges fit these: one
@@ -65,9 +68,17 @@ struct Span {
 };
 
 struct BlockState {
-    uint32_t win_v[kWinners], win_b[kWinners], win_d[kWinners];  // vertex, first out-edge, out-degree
+    union {
+        struct {  // push: the level's discoveries (vertex, first out-edge, out-degree)
+            uint32_t win_v[kWinners], win_b[kWinners], win_d[kWinners];
+        };
+        struct {  // pull, per warp: the chunk's vertices, those set aside, found bits
+            uint16_t items[kMaxWarps][32 * kPullWords];
+            uint16_t later[kMaxWarps][32 + 32 * kPullItems];
+            uint32_t found[kMaxWarps][kPullWords];
+        };
+    };
     uint4 solo[kSoloPieces];
-    uint32_t found[32 * kMaxWarps];  // pull: found bits of a warp's 32 words
     uint32_t win_cnt, win_end;       // appended; where the first append that did not fit starts
     uint32_t tot_ab[kMaxWarps], tot_u[kMaxWarps], tot_d[kMaxWarps], tot_disc[kMaxWarps], tot_deg[kMaxWarps];
     Span base;
@@ -509,154 +520,262 @@ __device__ __forceinline__ void solo_levels(const BfsArgs& a, BlockState& B, Run
     }
 }
 
+// The frontier of a pull level: its bitmap, read through L1 (nobody writes it
+// in this level), behind its summary in shared memory, which keeps most
+// probes of a small frontier off L2.
+struct Frontier {
+    const uint32_t* bits;
+    const uint32_t* summary;
+    uint32_t shift;
+    // Which of v[0..N) are in the frontier (entries may be kUnreached, which is
+    // not). All N bitmap loads are in flight together.
+    template <int N>
+    __device__ __forceinline__ void test(const uint32_t (&v)[N], bool (&hit)[N]) const {
+        bool may[N];
+        uint32_t word[N];
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            const uint32_t sb = (v[j] >> 5) >> shift;
+            may[j] = v[j] != kUnreached && (summary[v[j] != kUnreached ? sb >> 5 : 0u] >> (sb & 31)) & 1u;
+        }
+#pragma unroll
+        for (int j = 0; j < N; ++j) word[j] = may[j] ? bits[v[j] >> 5] : 0u;
+#pragma unroll
+        for (int j = 0; j < N; ++j) hit[j] = (word[j] >> (v[j] & 31)) & 1u;
+    }
+    // First of v[0..N) in the frontier, kUnreached if none.
+    template <int N>
+    __device__ __forceinline__ uint32_t first(const uint32_t (&v)[N]) const {
+        bool hit[N];
+        test(v, hit);
+        uint32_t x = kUnreached;
+#pragma unroll
+        for (int j = N - 1; j >= 0; --j)
+            if (hit[j]) x = v[j];
+        return x;
+    }
+};
+
 // Bottom-up level: a warp owns the words wi = warp + t * nwarps and takes them
-// 32 at a time: lane j loads word j's visited and has-in words, and the
-// unvisited vertices with in-neighbours of all 32 words are compacted into
-// one list (a warp scan of their counts) that the lanes take 32 at a time, so
-// no lane idles on a visited vertex. Each lane scans its vertex's
-// in-neighbours four at a time (independent loads) for at most kPullLaneScan
-// neighbours; the warp then finishes the longer lists together, 32 neighbours
-// per coalesced step, stopping at the first frontier neighbour; very long
-// lists go to the heavy queue. The next round's row bounds are loaded while
-// the current round is scanned. Found vertices set their bit in the warp's
-// word slots in shared memory; after the chunk lane j writes word j's visited
-// and frontier words. A
-// neighbour's frontier word is read, through L1 (nobody writes it in this
-// level), only when the summary in shared memory says it is non-empty.
-template <bool PARENTS, class InFrontier>
+// 16 at a time, two lanes per word (a half each): the unvisited vertices with
+// in-neighbours go into one list in shared memory that the lanes take 32 at a
+// time, so no lane idles on a visited vertex. (Finding a lane's vertex in the
+// words by shuffles and __fns instead cost more issue slots than the scan.)
+//
+// First every vertex tries its first four in-neighbours (those of highest
+// degree, DevGraph::heads: one aligned 16-byte load with the degree in its
+// spare bits, so no list bound is read; two vertices a lane, the next two's
+// loads in flight meanwhile). Most are settled by that: found, or their list
+// is done. The others are set aside, and lanes then take
+// them one by one, eight neighbours at a time, a lane that finishes taking the
+// next, so that no lane waits for the warp's longest scan in every round.
+// Lists with more than kPullWarpScan edges left are scanned by the whole warp,
+// very long ones by all warps after the level (heavy queue).
+//
+// Found vertices set their bit in the warp's word slots in shared memory;
+// after the chunk lane 2j writes word j's visited and frontier words.
+template <bool PARENTS>
 __device__ __forceinline__ void pull_level(const BfsArgs& a, BlockState& B, uint32_t level, uint32_t warp,
                                            uint32_t nwarps, uint32_t* fcur, uint32_t* fsum, unsigned long long* lvl,
-                                           InFrontier in_frontier, uint32_t& disc, uint32_t& deg) {
-    const uint32_t lane = threadIdx.x & 31;
+                                           const Frontier& front, uint32_t& disc, uint32_t& deg) {
+    const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1u;
     const DevGraph& g = a.g;
     const uint32_t W = (g.n + 31) / 32;
     const uint32_t tailMask = (g.n & 31) ? ((1u << (g.n & 31)) - 1) : 0xFFFFFFFFu;
     uint32_t longest = 0;
-    uint32_t* found_slots = B.found + (threadIdx.x & ~31u);
-    for (uint32_t t0 = 0; warp + t0 * nwarps < W; t0 += 32) {
-        const uint32_t wj = warp + (t0 + lane) * nwarps;
-        uint32_t visj = 0xFFFFFFFFu, unvj = 0;
-        if (wj < W) {
-            visj = __ldcg(&a.visited[wj]);
-            const uint32_t hj = g.has_in ? __ldg(&g.has_in[wj]) : 0xFFFFFFFFu;
-            unvj = ~visj & hj & (wj == W - 1 ? tailMask : 0xFFFFFFFFu);
-        }
-        // exclusive offsets of the words' items in the chunk's list
-        const uint32_t cj = __popc(unvj);
-        uint32_t incl = cj;
-#pragma unroll
-        for (uint32_t d = 1; d < 32; d <<= 1) {
-            const uint32_t o = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-            if (lane >= d) incl += o;
-        }
-        const uint32_t offj = incl - cj;
-        const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    const uint32_t w = threadIdx.x >> 5;
+    uint32_t* const found_slots = B.found[w];
+    uint16_t* const items = B.items[w];  // word slot << 5 | bit
+    uint16_t* const later = B.later[w];
+    // word `lane / 2` of the chunk at t0: visited word and the vertices to try
+    auto words = [&](uint32_t t0, uint32_t& vis) -> uint32_t {
+        const uint32_t wj = warp + (t0 + (lane >> 1)) * nwarps;
+        vis = 0xFFFFFFFFu;
+        if (wj >= W) return 0u;
+        vis = __ldcg(&a.visited[wj]);
+        const uint32_t hj = g.has_in ? __ldg(&g.has_in[wj]) : 0xFFFFFFFFu;
+        return ~vis & hj & (wj == W - 1 ? tailMask : 0xFFFFFFFFu);
+    };
+    uint32_t nvis, nunv = words(0, nvis);
+    for (uint32_t t0 = 0; warp + t0 * nwarps < W; t0 += kPullWords) {
+        const uint32_t vis = nvis, unv = nunv;
+        if (warp + (t0 + kPullWords) * nwarps < W) nunv = words(t0 + kPullWords, nvis);
+        uint32_t half = unv & (lane & 1 ? 0xFFFF0000u : 0xFFFFu);
+        uint32_t at = warp_incl(__popc(half));
+        const uint32_t total = __shfl_sync(0xFFFFFFFFu, at, 31);
         if (total == 0) continue;
-        found_slots[lane] = 0u;
+        at -= __popc(half);
+        if (lane < kPullWords) found_slots[lane] = 0u;
+        for (; half; half &= half - 1) items[at++] = (uint16_t)((lane >> 1) << 5 | (__ffs(half) - 1));
         __syncwarp();
-        // item idx -> (word slot, vertex); warp-uniform call
-        auto item = [&](uint32_t idx, uint32_t& slot, uint32_t& vtx) {
-            uint32_t lo = 0;
-#pragma unroll
-            for (uint32_t st = 16; st > 0; st >>= 1) {
-                const uint32_t o = __shfl_sync(0xFFFFFFFFu, offj, lo + st);
-                if (o <= idx) lo += st;
-            }
-            const uint32_t o = __shfl_sync(0xFFFFFFFFu, offj, lo);
-            const uint32_t um = __shfl_sync(0xFFFFFFFFu, unvj, lo);
-            slot = lo;
-            vtx = idx < total ? (warp + (t0 + lo) * nwarps) * 32 + __fns(um, 0, (int)(idx - o + 1)) : kUnreached;
+        auto vertex = [&](uint32_t code) { return (warp + (t0 + (code >> 5)) * nwarps) * 32 + (code & 31u); };
+        auto record = [&](uint32_t code, uint32_t u, uint32_t parent, uint32_t d) {
+            a.levels[u] = level;
+            if (PARENTS) a.parents[u] = parent;
+            atomicOr(&found_slots[code >> 5], 1u << (code & 31u));
+            ++disc;
+            deg += d;
         };
-        uint32_t nslot, nvtx;
-        item(lane, nslot, nvtx);
-        uint32_t npb = nvtx < g.n ? __ldg(&g.csr_ptrs[nvtx]) : 0u;
-        uint32_t npe = nvtx < g.n ? __ldg(&g.csr_ptrs[nvtx + 1]) : 0u;
-        for (uint32_t base = 0; base < total; base += 32) {
-            const uint32_t myslot = nslot, u = nvtx, pb = npb, pe = npe;
-            if (base + 32 < total) {
-                item(base + 32 + lane, nslot, nvtx);
-                npb = nvtx < g.n ? __ldg(&g.csr_ptrs[nvtx]) : 0u;
-                npe = nvtx < g.n ? __ldg(&g.csr_ptrs[nvtx + 1]) : 0u;
+        // the set-aside items later[0..cnt): lanes take them until none is left
+        auto drain = [&](uint32_t cnt) {
+            __syncwarp();
+            uint32_t code = 0, u = 0, p = 0, pe = 0, d = 0, next = 0;
+            bool busy = false;
+            for (;;) {
+                const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !busy);
+                if (idle && next < cnt) {
+                    const uint32_t k = next + __popc(idle & below);
+                    if (!busy && k < cnt) {
+                        code = later[k];
+                        u = vertex(code);
+                        p = __ldg(&g.csr_ptrs[u]);
+                        pe = __ldg(&g.csr_ptrs[u + 1]);
+                        d = pe - p;
+                        p += 4;
+                        busy = true;
+                    }
+                    next = min(cnt, next + __popc(idle));
+                }
+                if (!__any_sync(0xFFFFFFFFu, busy)) break;
+                if (busy) {
+                    // two aligned quads (the lists are padded to whole quads)
+                    const uint32_t q = p & ~3u;
+                    const uint4 x = __ldg(reinterpret_cast<const uint4*>(g.csr_ids + q));
+                    const uint4 y = q + 4 < pe ? __ldg(reinterpret_cast<const uint4*>(g.csr_ids + q + 4))
+                                               : make_uint4(0u, 0u, 0u, 0u);
+                    uint32_t v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+                    for (uint32_t j = 0; j < 8; ++j)
+                        if (q + j < p || q + j >= pe) v[j] = kUnreached;
+                    const uint32_t parent = front.first(v);
+                    p = q + 8;
+                    if (parent != kUnreached) record(code, u, parent, d);
+                    busy = parent == kUnreached && p < pe;
+                }
             }
-            bool found = false;
-            uint32_t parent = kUnreached, p = pb;
-            if (u < g.n) {
-                const uint32_t cap = pb + min(pe - pb, kPullLaneScan);
-                for (; p < cap && !found; p += kPullUnroll) {
-                    uint32_t v[kPullUnroll];
-                    bool f[kPullUnroll];
+            __syncwarp();
+        };
+        uint32_t ncode[kPullItems], waiting = 0;
+        uint4 nhead[kPullItems];
+        auto fetch = [&](uint32_t base) {
 #pragma unroll
-                    for (uint32_t j = 0; j < kPullUnroll; ++j)
-                        v[j] = p + j < pe ? __ldg(&g.csr_ids[p + j]) : kUnreached;
+            for (uint32_t k = 0; k < kPullItems; ++k) {
+                const uint32_t idx = base + 32 * k + lane;
+                ncode[k] = 0;
+                nhead[k] = make_uint4(0u, 0u, 0u, 0u);  // an empty list
+                if (idx < total) {
+                    ncode[k] = items[idx];
+                    nhead[k] = __ldg(&g.heads[vertex(ncode[k])]);
+                }
+            }
+        };
+        fetch(0);
+        for (uint32_t base = 0; base < total; base += 32 * kPullItems) {
+            uint32_t code[kPullItems], d[kPullItems], parent[kPullItems], v[kPullItems][4];
 #pragma unroll
-                    for (uint32_t j = 0; j < kPullUnroll; ++j) f[j] = v[j] != kUnreached && in_frontier(v[j]);
+            for (uint32_t k = 0; k < kPullItems; ++k) {
+                code[k] = ncode[k];
+                const uint4 h = nhead[k];
+                d[k] = head_degree(h);
+                const uint32_t x[4] = {h.x, h.y, h.z, h.w};
 #pragma unroll
-                    for (uint32_t j = 0; j < kPullUnroll; ++j) {
-                        if (!found && f[j]) {
-                            found = true;
-                            parent = v[j];
+                for (uint32_t j = 0; j < 4; ++j) v[k][j] = d[k] > j ? x[j] & kHeadId : kUnreached;
+            }
+            if (base + 32 * kPullItems < total) fetch(base + 32 * kPullItems);
+            // Two neighbours, then two more: 32 lanes' probes are 32 L1 lines
+            // (one a clock), so probes past the first hit cost more than the
+            // round trip that testing all four at once would save.
+            {
+                uint32_t x[2 * kPullItems];
+                bool hit[2 * kPullItems];
+#pragma unroll
+                for (uint32_t k = 0; k < kPullItems; ++k) {
+                    x[2 * k] = v[k][0];
+                    x[2 * k + 1] = v[k][1];
+                }
+                front.test(x, hit);
+                bool more = false;
+#pragma unroll
+                for (uint32_t k = 0; k < kPullItems; ++k) {
+                    parent[k] = hit[2 * k] ? x[2 * k] : (hit[2 * k + 1] ? x[2 * k + 1] : kUnreached);
+                    const bool on = parent[k] == kUnreached && d[k] > 2;
+                    more |= on;
+                    x[2 * k] = on ? v[k][2] : kUnreached;
+                    x[2 * k + 1] = on ? v[k][3] : kUnreached;
+                }
+                if (more) {
+                    front.test(x, hit);
+#pragma unroll
+                    for (uint32_t k = 0; k < kPullItems; ++k) {
+                        if (hit[2 * k + 1]) parent[k] = x[2 * k + 1];
+                        if (hit[2 * k]) parent[k] = x[2 * k];
+                    }
+                }
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < kPullItems; ++k) {
+                const uint32_t u = vertex(code[k]);
+                uint32_t p = 0, pe = 0;
+                const bool is_long = d[k] > kPullWarpScan + 4;
+                if (d[k] >= kHeadDegreeMax || (is_long && parent[k] == kUnreached)) {
+                    p = __ldg(&g.csr_ptrs[u]);
+                    pe = __ldg(&g.csr_ptrs[u + 1]);
+                    d[k] = pe - p;
+                    p += 4;
+                    if (parent[k] != kUnreached) p = pe;  // settled
+                }
+                // Very long lists go to the heavy queue (all warps split them
+                // after the level barrier).
+                if (p < pe && pe - p > a.heavy_min) {
+                    const uint32_t chunks = (pe - p + kHeavyChunk - 1) / kHeavyChunk;
+                    const uint64_t hs = atomicAdd(&lvl[3], (unsigned long long)((1ull << kQShift) | chunks));
+                    const uint32_t idx = (uint32_t)(hs >> kQShift);
+                    if (idx < a.heavy_cap) {
+                        a.heavy[idx] = make_uint4(u, p, pe, (uint32_t)(hs & kQUnitMask));
+                        p = pe;  // handed over
+                    } else {
+                        set_error(a.ctr, BLEST_ERR_DEVICE_INDEX);  // capacity is sized so this cannot happen
+                    }
+                }
+                // Long lists: the whole warp scans them, one vertex at a time.
+                for (uint32_t rest = __ballot_sync(0xFFFFFFFFu, p < pe); rest; rest &= rest - 1) {
+                    const uint32_t ln = __ffs(rest) - 1;
+                    const uint32_t q0 = __shfl_sync(0xFFFFFFFFu, p, ln);
+                    const uint32_t q1 = __shfl_sync(0xFFFFFFFFu, pe, ln);
+                    longest = max(longest, q1 - q0);
+                    uint32_t hitv = kUnreached;
+                    for (uint32_t qb = q0; qb < q1 && hitv == kUnreached; qb += 128) {
+                        uint32_t x[4];
+#pragma unroll
+                        for (uint32_t j = 0; j < 4; ++j) {
+                            const uint32_t idx = qb + 32 * j + lane;
+                            x[j] = idx < q1 ? __ldg(&g.csr_ids[idx]) : kUnreached;
                         }
+                        const uint32_t mine = front.first(x);
+                        const uint32_t hb = __ballot_sync(0xFFFFFFFFu, mine != kUnreached);
+                        if (hb) hitv = __shfl_sync(0xFFFFFFFFu, mine, __ffs(hb) - 1);
                     }
+                    if (lane == ln) parent[k] = hitv;
                 }
+                if (parent[k] != kUnreached) record(code[k], u, parent[k], d[k]);
+                const bool aside = parent[k] == kUnreached && d[k] > 4 && !is_long;
+                const uint32_t am = __ballot_sync(0xFFFFFFFFu, aside);
+                if (aside) later[waiting + __popc(am & below)] = (uint16_t)code[k];
+                waiting += __popc(am);
             }
-            // Very long lists go to the heavy queue (all warps split them
-            // after the level barrier).
-            if (!found && p < pe && pe - p > a.heavy_min) {
-                const uint32_t chunks = (pe - p + kHeavyChunk - 1) / kHeavyChunk;
-                const uint64_t hs = atomicAdd(&lvl[3], (unsigned long long)((1ull << kQShift) | chunks));
-                const uint32_t idx = (uint32_t)(hs >> kQShift);
-                if (idx < a.heavy_cap) {
-                    a.heavy[idx] = make_uint4(u, p, pe, (uint32_t)(hs & kQUnitMask));
-                    p = pe;  // handed over
-                } else {
-                    set_error(a.ctr, BLEST_ERR_DEVICE_INDEX);  // capacity is sized so this cannot happen
-                }
-            }
-            // Long lists: the whole warp scans them, one vertex at a time.
-            for (uint32_t rest = __ballot_sync(0xFFFFFFFFu, !found && p < pe); rest; rest &= rest - 1) {
-                const uint32_t ln = __ffs(rest) - 1;
-                const uint32_t q0 = __shfl_sync(0xFFFFFFFFu, p, ln);
-                const uint32_t q1 = __shfl_sync(0xFFFFFFFFu, pe, ln);
-                longest = max(longest, q1 - q0);
-                uint32_t hitv = kUnreached;
-                for (uint32_t qb = q0; qb < q1; qb += 32) {
-                    const uint32_t idx = qb + lane;
-                    const uint32_t v = idx < q1 ? __ldg(&g.csr_ids[idx]) : kUnreached;
-                    const uint32_t hb = __ballot_sync(0xFFFFFFFFu, v != kUnreached && in_frontier(v));
-                    if (hb) {
-                        hitv = __shfl_sync(0xFFFFFFFFu, v, __ffs(hb) - 1);
-                        break;
-                    }
-                }
-                if (lane == ln && hitv != kUnreached) {
-                    found = true;
-                    parent = hitv;
-                }
-            }
-            if (found) {
-                a.levels[u] = level;
-                if (PARENTS) a.parents[u] = parent;
-                ++disc;
-                deg += pe - pb;
-            }
-            // this round's found bits, merged per word slot by a warp
-            // reduction: one store per distinct slot (lanes of one word
-            // would otherwise collide on the same shared-memory word)
-            for (uint32_t pending = __ballot_sync(0xFFFFFFFFu, found); pending;) {
-                const uint32_t slot = __shfl_sync(0xFFFFFFFFu, myslot, __ffs(pending) - 1);
-                const bool mine = found && myslot == slot;
-                const uint32_t bits = __reduce_or_sync(0xFFFFFFFFu, mine ? 1u << (u & 31) : 0u);
-                if (lane == 0) found_slots[slot] |= bits;
-                pending &= ~__ballot_sync(0xFFFFFFFFu, mine);
+            if (waiting >= 32) {
+                drain(waiting);
+                waiting = 0;
             }
         }
-        __syncwarp();
-        // write back the chunk's words (lane j: word j)
-        const uint32_t nb = found_slots[lane];
+        drain(waiting);
+        // write back the chunk's words (lanes 2j: word j)
+        const uint32_t nb = lane & 1 ? 0u : found_slots[lane >> 1];
         __syncwarp();
         if (nb) {
+            const uint32_t wj = warp + (t0 + (lane >> 1)) * nwarps;
             fcur[wj] = nb;
-            a.visited[wj] = visj | nb;
+            a.visited[wj] = vis | nb;
             mark_summary(a, fsum, wj);
         }
     }
@@ -666,9 +785,9 @@ __device__ __forceinline__ void pull_level(const BfsArgs& a, BlockState& B, uint
 
 // The heavy lists of a pull level: every warp takes an equal share of their
 // pieces.
-template <bool PARENTS, class InFrontier>
+template <bool PARENTS>
 __device__ __forceinline__ void heavy_level(const BfsArgs& a, uint64_t hq, uint32_t level, uint32_t warp,
-                                            uint32_t nwarps, uint32_t* fcur, uint32_t* fsum, InFrontier in_frontier,
+                                            uint32_t nwarps, uint32_t* fcur, uint32_t* fsum, const Frontier& front,
                                             uint32_t& disc, uint32_t& deg) {
     const uint32_t lane = threadIdx.x & 31;
     const DevGraph& g = a.g;
@@ -691,9 +810,9 @@ __device__ __forceinline__ void heavy_level(const BfsArgs& a, uint64_t hq, uint3
         for (uint32_t base = q0; base < q1 && hitv == kUnreached; base += 32) {
             if (__ldcg(&a.visited[w]) & b) break;  // another piece found it
             const uint32_t idx = base + lane;
-            const uint32_t v = idx < q1 ? __ldg(&g.csr_ids[idx]) : kUnreached;
-            const uint32_t hb = __ballot_sync(0xFFFFFFFFu, v != kUnreached && in_frontier(v));
-            if (hb) hitv = __shfl_sync(0xFFFFFFFFu, v, __ffs(hb) - 1);
+            const uint32_t v[1] = {idx < q1 ? __ldg(&g.csr_ids[idx]) : kUnreached};
+            const uint32_t hb = __ballot_sync(0xFFFFFFFFu, front.first(v) != kUnreached);
+            if (hb) hitv = __shfl_sync(0xFFFFFFFFu, v[0], __ffs(hb) - 1);
         }
         if (hitv != kUnreached && lane == 0 && !(atomicOr(&a.visited[w], b) & b)) {
             a.levels[hu] = level;
@@ -941,26 +1060,21 @@ __device__ __forceinline__ void lists_run(const BfsArgs& a) {
                 s.size = span_of(B.val[0], B.val[4]);
             }
         } else {
-            const uint32_t* fprev = bitmap_of(a, gen);
+            const Frontier front{bitmap_of(a, gen), s_sum, a.sum_shift};
             const uint32_t* sprev = summary_of(a, gen);
             for (uint32_t i = threadIdx.x; i < a.sum_words; i += blockDim.x) s_sum[i] = __ldcg(&sprev[i]);
             ++gen;
             clear_next();
             uint32_t* fcur = bitmap_of(a, gen);
             uint32_t* fsum = summary_of(a, gen);
-            auto in_frontier = [&](uint32_t v) -> bool {
-                const uint32_t sb = (v >> 5) >> a.sum_shift;
-                if (!((s_sum[sb >> 5] >> (sb & 31)) & 1u)) return false;
-                return (fprev[v >> 5] >> (v & 31)) & 1u;
-            };
             __syncthreads();
-            pull_level<PARENTS>(a, B, level, warp, nwarps, fcur, fsum, lvl, in_frontier, disc, deg);
+            pull_level<PARENTS>(a, B, level, warp, nwarps, fcur, fsum, lvl, front, disc, deg);
             if (tid == 0) c->pull_levels++;
             if (!level_end(a, B, lvl, true, disc, deg)) return;
             if (B.val[3]) {
                 const uint64_t hq = B.val[3];
                 disc = deg = 0;
-                heavy_level<PARENTS>(a, hq, level, warp, nwarps, fcur, fsum, in_frontier, disc, deg);
+                heavy_level<PARENTS>(a, hq, level, warp, nwarps, fcur, fsum, front, disc, deg);
                 if (!level_end(a, B, lvl, true, disc, deg)) return;
             }
         }

@@ -395,6 +395,18 @@ __global__ void out_fill_kernel(DevGraph g, const uint32_t* ptrs, uint32_t* ids)
     }
 }
 
+__global__ void list_heads_kernel(DevGraph g, uint4* heads) {
+    const uint32_t nth = gridDim.x * blockDim.x;
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < g.n; v += nth) {
+        const uint32_t b = __ldg(&g.csr_ptrs[v]), e = __ldg(&g.csr_ptrs[v + 1]);
+        uint32_t h[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k)
+            h[k] = (e - b > k ? __ldg(&g.csr_ids[b + k]) : 0u) | ((min(e - b, kHeadDegreeMax) >> (4 * k)) & 15u) << 28;
+        heads[v] = make_uint4(h[0], h[1], h[2], h[3]);
+    }
+}
+
 }  // namespace dev
 
 namespace {
@@ -554,6 +566,15 @@ bool tiles_symmetric_device(const dev::DevGraph& d, cudaStream_t s) {
     BLEST_CUDA(cudaMemcpyAsync(&h, out, sizeof(Out), cudaMemcpyDeviceToHost, s));
     BLEST_CUDA(cudaStreamSynchronize(s));
     return !h.bad && h.edges == d.nnz;
+}
+
+void list_heads_device(const dev::DevGraph& d, uint4* heads, cudaStream_t s) {
+    int dev = 0, sms = 0;
+    BLEST_CUDA(cudaGetDevice(&dev));
+    BLEST_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    dev::list_heads_kernel<<<sms * 8, 256, 0, s>>>(d, heads);
+    BLEST_CUDA(cudaGetLastError());
+    BLEST_CUDA(cudaStreamSynchronize(s));
 }
 
 bool out_lists_device(const dev::DevGraph& d, cudaStream_t s, OutLists& out) {

@@ -47,8 +47,19 @@ struct DevGraph {
     // pull lists themselves when the graph is symmetric. Null: not kept.
     const uint32_t* out_ptrs;  // n + 1
     const uint32_t* out_ids;
+    // First four ids of each pull list in the low 28 bits, its length in the
+    // high 4 bits of the four (head_degree); kept with out_ptrs.
+    const uint4* heads;
     uint32_t piece_cap;        // BFS queue entries: one per vertex, and one more per kBfsPieceEdges edges for long lists
 };
+
+// DevGraph::heads: ids are below 2^28 (checked when a graph is made); the
+// high bits, x's first, hold min(list length, kHeadDegreeMax).
+constexpr uint32_t kHeadId = (1u << 28) - 1;
+constexpr uint32_t kHeadDegreeMax = 0xFFFF;
+__host__ __device__ __forceinline__ uint32_t head_degree(const uint4& h) {
+    return (h.x >> 28) | (h.y >> 28) << 4 | (h.z >> 28) << 8 | (h.w >> 28) << 12;
+}
 
 // Most edges of one piece of the BFS push queue.
 constexpr uint32_t kBfsPieceEdges = 128;

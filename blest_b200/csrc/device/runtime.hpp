@@ -167,6 +167,8 @@ struct OutLists {
     uint32_t* ids = nullptr;
     uint32_t edges = 0;
 };
+// DevGraph::heads of the pull lists.
+void list_heads_device(const dev::DevGraph& d, uint4* heads, cudaStream_t s);
 bool out_lists_device(const dev::DevGraph& d, cudaStream_t s, OutLists& out);
 void mbfs_scratch_free(void* p);
 // Allocate the multi-source BFS state of `words` 32-bit words per vertex now.
