@@ -9,21 +9,29 @@
 // unreached).
 //
 // Per level, for a group of up to 32 * WORDS sources:
-//  - expand: push over BVSS tiles of the rsets with frontier bits (a warp
+//  - first half: push over BVSS tiles of the rsets with frontier bits (a warp
 //    per 32-tile chunk of one rset; the rset's 8 column frontier words are
 //    shared by shuffle; next[row] |= OR of the hit columns' words, by
-//    atomicOr), or pull over the degree-ordered CSR (next[v] = OR of the
-//    in-neighbours' frontier words, stopping once every bit v still needs
-//    is covered);
-//  - sweep: new = next & ~visited; visited |= new; the new bits are level
-//    L's frontier, kept in history slot L % hist_slots; rsets with new bits
-//    queued for a push.
+//    atomicOr); and the long in-lists of graphs that pull, in pieces, also
+//    into `next`. Left out, with its barrier, when no graph needs it;
+//  - second half, over the words of the graphs with a frontier: graphs that
+//    pull scan their short in-lists here (degree-ordered; stopping once every
+//    bit the vertex still needs is covered), the others take next & ~visited;
+//    the new bits go into visited and are level L's frontier, kept in
+//    history slot L % hist_slots; rsets with new bits are queued for a push.
 // Levels are written once per (source, vertex), after the group's last
 // level, by one pass that reads the vertex's history slots and writes
 // every source row of 32 consecutive vertices at a time (full 128-byte
 // rows, no "unreached" pre-fill and no partial-sector writes per level).
 // When a group has more levels than slots, the oldest slots are written
 // out first (their sectors then take two partial writes).
+//
+// What bounds it: pull levels by the L1 (a lane's gather costs a cycle of it
+// whatever its width: RMAT-20 with 128 sources scans about 31 M neighbours in
+// its biggest level, 190 us, at 0.25 id loads and one 16-byte gather each),
+// sparse push levels by the tiles of whole sets, the write-out by HBM.
+// RMAT-20 x 256 sources, device time: 1846 -> 1410 us (biggest pull level 237
+// -> 192, the next ones 84 / 50 -> 55 / 29, write-out of 540 MB 280 -> 170).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -77,7 +85,7 @@ struct MbfsArgs {
     const uint32_t* word_part;
     MbfsPart part0;
     const uint32_t* sources;   // local source ids, per part from src_base
-    uint32_t* part_nf;         // 2 slots x nparts: vertices found per part at the last two levels
+    uint32_t* part_nf;         // 3 slots x nparts: vertices found per part (slot = level % 3)
     blest_level_trace* trace;  // optional: one record per level of every group
     // Single-graph runs only: when set, source i's levels go to rows[i]
     // (one caller buffer of n words per source) instead of part0.levels.
@@ -213,6 +221,24 @@ __device__ __forceinline__ Bits<WORDS> load_bits(const uint32_t* a, uint32_t v) 
     return b;
 }
 
+// The same through L1, for words that nobody writes while they are read (the
+// previous level's frontier): neighbours of high degree, first in every list,
+// are read again and again.
+template <int WORDS>
+__device__ __forceinline__ Bits<WORDS> load_frontier(const uint32_t* a, uint32_t v) {
+    Bits<WORDS> b;
+    if constexpr (WORDS == 4) {
+        const uint4 x = reinterpret_cast<const uint4*>(a)[v];
+        b.w[0] = x.x; b.w[1] = x.y; b.w[2] = x.z; b.w[3] = x.w;
+    } else if constexpr (WORDS == 2) {
+        const uint2 x = reinterpret_cast<const uint2*>(a)[v];
+        b.w[0] = x.x; b.w[1] = x.y;
+    } else {
+        b.w[0] = a[v];
+    }
+    return b;
+}
+
 template <int WORDS>
 __device__ __forceinline__ void store_bits(uint32_t* a, uint32_t v, const Bits<WORDS>& b) {
     if constexpr (WORDS == 4) {
@@ -226,19 +252,28 @@ __device__ __forceinline__ void store_bits(uint32_t* a, uint32_t v, const Bits<W
 
 // OR of the frontier bits of in-neighbours csr_ids[q, qe) into acc, limited
 // to `need`; four neighbours' loads in flight at a time; stops once acc
-// covers need.
+// covers need. Ids come as aligned quads (the array is padded to whole ones):
+// each lane scans its own list, so a load instruction costs one L1 cycle per
+// lane whatever its width, and four 4-byte id loads cost as much as the four
+// gathers they lead to.
 template <int WORDS>
 __device__ __forceinline__ void scan_in_list(const MbfsArgs& a, const uint32_t* frontier, uint32_t q, uint32_t qe,
                                              const uint32_t (&need)[WORDS], uint32_t (&acc)[WORDS]) {
-    for (; q < qe; q += 4) {
-        uint32_t u[4];
+    const uint4* ids = reinterpret_cast<const uint4*>(a.g.csr_ids);
+    uint4 x = __ldg(ids + (q >> 2));
+    for (uint32_t q0 = q & ~3u; q0 < qe; q0 += 4) {
+        uint32_t u[4] = {x.x, x.y, x.z, x.w};
+        // the next quad is on its way while this one's words are gathered (a
+        // warp's time here is its longest list's chain of round trips)
+        if (q0 + 4 < qe) x = __ldg(ids + (q0 >> 2) + 1);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) u[j] = q + j < qe ? __ldg(&a.g.csr_ids[q + j]) : 0xFFFFFFFFu;
+        for (int j = 0; j < 4; ++j)
+            if (q0 + j < q || q0 + j >= qe) u[j] = 0xFFFFFFFFu;
         Bits<WORDS> f[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             if (u[j] != 0xFFFFFFFFu) {
-                f[j] = load_bits<WORDS>(frontier, u[j]);
+                f[j] = load_frontier<WORDS>(frontier, u[j]);
             } else {
 #pragma unroll
                 for (int w = 0; w < WORDS; ++w) f[j].w[w] = 0u;
@@ -257,6 +292,78 @@ __device__ __forceinline__ void scan_in_list(const MbfsArgs& a, const uint32_t* 
 template <int WORDS>
 __device__ __forceinline__ uint32_t* hist_slot(const MbfsArgs& a, uint32_t level) {
     return a.hist + (size_t)(level & (a.hist_slots - 1)) * a.g.n * WORDS;
+}
+
+// Most levels a group may have for write_bytes: they are written as signed
+// bytes first, -1 for unreached (and at most 64 history slots hold them all).
+constexpr uint32_t kByteLevels = 64;
+
+// All levels 0..top of a word's 32 vertices (lane = vertex v, local id lv) to
+// the group's rows, each once. The levels are kept bit-sliced for all WORDS
+// source words (one 16-byte load per level), then spread to one byte per
+// source, four sources at a time: a multiply and a mask per bit plane, and
+// one byte permute with sign extension per row, instead of collecting six
+// planes' bits and two masks row by row (~25 instructions a row; the pass of
+// an RMAT-20 group of 128 took 280 us for 540 MB).
+template <int WORDS>
+__device__ __forceinline__ void write_bytes(const MbfsArgs& a, const MbfsPart& P, uint32_t v, bool in, uint32_t lv,
+                                            uint32_t rows, uint32_t s0, uint32_t top) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t plane[6][WORDS], found[WORDS];
+#pragma unroll
+    for (int w = 0; w < WORDS; ++w) {
+        found[w] = 0u;
+#pragma unroll
+        for (int j = 0; j < 6; ++j) plane[j][w] = 0u;
+    }
+    for (uint32_t L = 0; L <= top; ++L) {
+        Bits<WORDS> f;
+        if (in) {
+            f = load_bits<WORDS>(hist_slot<WORDS>(a, L), v);
+        } else {
+#pragma unroll
+            for (int w = 0; w < WORDS; ++w) f.w[w] = 0u;
+        }
+#pragma unroll
+        for (int w = 0; w < WORDS; ++w) {
+            found[w] |= f.w[w];
+#pragma unroll
+            for (int j = 0; j < 6; ++j)
+                if ((L >> j) & 1u) plane[j][w] |= f.w[w];
+        }
+    }
+    const uint32_t planes = 32 - __clz(top);  // uniform; 0 when top is 0
+    auto spread = [](uint32_t bits) { return ((bits & 0xFu) * 0x00204081u) & 0x01010101u; };
+#pragma unroll
+    for (int w = 0; w < WORDS; ++w) {
+        const uint32_t rw = rows > 32u * w ? min(32u, rows - 32u * w) : 0u;
+        if (rw == 0) break;
+        // with a rows table, lane j holds the buffer of the word's j-th source
+        uint32_t* mine = nullptr;
+        if (a.rows && lane < rw) mine = a.rows[s0 + 32u * w + lane];
+        uint32_t* dst = a.rows ? nullptr : P.levels + (uint64_t)(s0 + 32u * w) * P.n + lv;
+        for (uint32_t b = 0; b < rw; b += 4) {
+            uint32_t x = spread(~found[w] >> b) * 0xFFu;
+#pragma unroll
+            for (int j = 0; j < 6; ++j)
+                if ((uint32_t)j < planes) x |= spread(plane[j][w] >> b) << j;
+#pragma unroll
+            for (uint32_t t = 0; t < 4; ++t) {
+                if (b + t >= rw) break;
+                // byte t sign-extended (__byte_perm has no sign mode)
+                uint32_t lvl;
+                asm("prmt.b32 %0, %1, 0, %2;" : "=r"(lvl) : "r"(x), "r"(t * 0x1111u | 0x8880u));
+                if (a.rows) {
+                    uint32_t* const d = reinterpret_cast<uint32_t*>(
+                        __shfl_sync(0xFFFFFFFFu, reinterpret_cast<unsigned long long>(mine), b + t));
+                    if (in) __stcs(d + lv, lvl);
+                } else {
+                    if (in) __stcs(dst, lvl);
+                    dst += P.n;
+                }
+            }
+        }
+    }
 }
 
 // Levels [lo, min(hi, part_last[p])] of the group starting at source s0
@@ -279,6 +386,10 @@ __device__ __forceinline__ void write_levels(const MbfsArgs& a, uint32_t warp, u
         const bool in = lv < P.n;
         const uint32_t rows = group_rows(P, s0, a.group_width);
         const uint32_t top = min(hi, __ldcg(&a.part_last[p]));
+        if (final && lo == 0 && top < kByteLevels) {
+            write_bytes<WORDS>(a, P, v, in, lv, rows, s0, top);
+            return;
+        }
 #pragma unroll
         for (int w = 0; w < WORDS; ++w) {
             const uint32_t rw = rows > 32u * w ? min(32u, rows - 32u * w) : 0u;
@@ -321,8 +432,55 @@ __device__ __forceinline__ void write_levels(const MbfsArgs& a, uint32_t warp, u
     });
 }
 
+// What a graph does at a level.
+enum PartMode : uint8_t { kIdle = 0, kPush = 1, kPull = 2 };
+constexpr uint32_t kModeParts = 1024;  // graphs whose mode a block keeps in shared memory
+constexpr uint32_t kQueueBuf = 64;     // rsets a warp gathers before it appends them to the queue
+
+struct MbfsShared {
+    uint8_t mode[kModeParts];
+    uint32_t rset[16][kQueueBuf], units[16][kQueueBuf];
+    uint32_t cnt[16];
+    uint32_t halves;  // some graph needs the level's first half
+    unsigned long long nf, queue;
+};
+
+__device__ __forceinline__ uint32_t part_mode(const MbfsArgs& a, const MbfsPart& P, uint32_t found) {
+    return found == 0 ? kIdle : ((double)found > (double)P.n * a.pull_fraction ? kPull : kPush);
+}
+
+// Append the warp's k buffered rsets to the queue with one atomic (one per
+// word of a sweep put up to n / 32 of them on one counter, about a
+// nanosecond each: 33 us a level for a million vertices).
+__device__ __forceinline__ void flush_rsets(const MbfsArgs& a, MbfsShared& S, uint32_t k, unsigned long long* counter,
+                                            uint32_t* q_rset, uint32_t* q_off) {
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __syncwarp();
+    for (uint32_t i0 = 0; i0 < k; i0 += 32) {
+        const bool in = i0 + lane < k;
+        const uint32_t r = in ? S.rset[w][i0 + lane] : 0u;
+        const uint64_t mine = in ? (1ull << kQShift) | S.units[w][i0 + lane] : 0ull;
+        const uint64_t incl = warp_inclusive_scan64(mine);
+        uint64_t b0 = 0;
+        if (lane == 31) b0 = atomicAdd(counter, (unsigned long long)incl);
+        b0 = __shfl_sync(0xFFFFFFFFu, b0, 31);
+        if (in) {
+            const uint64_t ex = b0 + incl - mine;
+            const uint32_t e = (uint32_t)(ex >> kQShift);
+            if (e < a.qreg) {
+                q_rset[e] = r;
+                q_off[e] = (uint32_t)(ex & kQUnitMask);
+            } else {
+                set_error(a.ctr, BLEST_ERR_DEVICE_INDEX);
+            }
+        }
+    }
+    __syncwarp();
+}
+
 template <int WORDS>
 __global__ void __launch_bounds__(512, 2) mbfs_persistent_kernel(MbfsArgs a) {
+    __shared__ MbfsShared S;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t nth = gridDim.x * blockDim.x;
@@ -344,10 +502,10 @@ __global__ void __launch_bounds__(512, 2) mbfs_persistent_kernel(MbfsArgs a) {
         for (uint32_t p = tid; p < a.nparts; p += nth) a.part_last[p] = 0u;
         uint32_t base = 0;  // first level not yet written to the output
         if (tid == 0) {
-            c->aux[0] = c->aux[1] = 0;  // push queue counters (2 slots)
-            c->aux[4] = c->aux[5] = 0;  // new-frontier vertex counts (2 slots)
+            c->aux[0] = c->aux[1] = c->aux[2] = 0;  // push queue counters (3 slots)
+            c->aux[3] = c->aux[4] = c->aux[5] = 0;  // new-frontier vertex counts (3 slots)
         }
-        for (uint32_t i = tid; i < 2 * a.nparts; i += nth) a.part_nf[i] = 0u;
+        for (uint32_t i = tid; i < 3 * a.nparts; i += nth) a.part_nf[i] = 0u;
         if (!barrier()) return;
         // ---- seeds: pair t = (part t / width, slot t % width); the sources'
         // rsets are queued in slot 0 (duplicates are harmless)
@@ -396,27 +554,49 @@ __global__ void __launch_bounds__(512, 2) mbfs_persistent_kernel(MbfsArgs a) {
                 }
             }
             const uint64_t ws = warp_sum64(seeded);
-            if (lane == 0 && ws) atomicAdd(&c->aux[4], (unsigned long long)ws);
+            if (lane == 0 && ws) atomicAdd(&c->aux[3], (unsigned long long)ws);
         }
         if (!barrier()) return;
 
+        uint64_t found = 0;  // vertices found up to the last level (once per level)
         for (uint32_t level = 1;; ++level) {
-            const uint32_t slot = (level - 1) & 1;  // queue/counts produced by the previous sweep
-            const uint64_t nf = ld_relaxed64(&c->aux[4 + slot]);
+            const uint32_t slot = (level - 1) & 1;  // queue filled by the previous level (the coming one fills slot ^ 1)
+            // Counts, three slots in turn: those of the last level, those of
+            // this one (zero since the last level, whose barrier no add can
+            // overtake) and the next one's, zeroed meanwhile.
+            const uint32_t cin = (level - 1) % 3, cout = level % 3, cnext = (level + 1) % 3;
+            // The level's counts, read once per block: a word that every warp
+            // of the grid reads costs its L2 slice about a nanosecond a read.
+            // Per graph: idle (it found nothing at level - 1), pull (that
+            // frontier holds more than n * pull_fraction vertices) or push.
+            const uint32_t* nfp = a.part_nf + cin * a.nparts;
+            if (threadIdx.x == 0) {
+                S.nf = ld_relaxed64(&c->aux[3 + cin]);
+                S.queue = ld_relaxed64(&c->aux[cin]);
+            }
+            if (threadIdx.x == 0) S.halves = 0;
+            __syncthreads();
+            for (uint32_t p = threadIdx.x; p < a.nparts; p += blockDim.x) {
+                const MbfsPart P = load_part(a, p);
+                const uint32_t m = part_mode(a, P, __ldcg(&nfp[p]));
+                if (p < kModeParts) S.mode[p] = (uint8_t)m;
+                if (m == kPush || (m == kPull && P.ccount)) S.halves = 1;
+            }
+            __syncthreads();
+            auto mode_of = [&](uint32_t p, const MbfsPart& P) -> uint32_t {
+                return p < kModeParts ? (uint32_t)S.mode[p] : part_mode(a, P, __ldcg(&nfp[p]));
+            };
+            const uint64_t nf = S.nf;
             if (a.trace && tid == 0 && c->trace_records < BLEST_TRACE_CAPACITY) {
                 // direction summary: 1 push, 2 pull, 3 both (several graphs)
                 uint32_t dirs = 0;
-                for (uint32_t p = 0; p < a.nparts && dirs != 3; ++p) {
-                    const MbfsPart P = load_part(a, p);
-                    const uint32_t x = __ldcg(&a.part_nf[slot * a.nparts + p]);
-                    if (x) dirs |= (double)x > (double)P.n * a.pull_fraction ? 2u : 1u;
-                }
+                for (uint32_t p = 0; p < a.nparts && dirs != 3; ++p) dirs |= mode_of(p, load_part(a, p));
                 blest_level_trace& t = a.trace[c->trace_records++];
                 t.start_ns = global_ns();
                 t.level = nf ? level : 0;
                 t.direction = dirs;
                 t.frontier = nf;
-                t.work_units = ld_relaxed64(&c->aux[slot]) & kQUnitMask;
+                t.work_units = S.queue & kQUnitMask;
                 t.longest_scan = grp;
                 t.sweep_ns = 0;
             }
@@ -428,56 +608,28 @@ __global__ void __launch_bounds__(512, 2) mbfs_persistent_kernel(MbfsArgs a) {
             // slot level % hist_slots still holds unwritten level `base`:
             // write levels [base, level) out first (the sweep that reuses
             // the slot comes after the next barrier)
-            if (level - base == a.hist_slots) {
+            const bool written = level - base == a.hist_slots;
+            if (written) {
                 write_levels<WORDS>(a, warp, nwarps, s0, base, level - 1, false);
                 base = level;
             }
 
             if (tid == 0) {
-                c->aux[slot ^ 1] = 0;      // queue slot the coming sweep fills
-                c->aux[4 + (slot ^ 1)] = 0;
+                c->aux[cnext] = 0;
+                c->aux[3 + cnext] = 0;
             }
-            for (uint32_t p = tid; p < a.nparts; p += nth) a.part_nf[(slot ^ 1) * a.nparts + p] = 0u;
-            // Per graph: active = it found vertices at level L-1; it pulls
-            // when that frontier holds more than n * pull_fraction vertices.
-            const uint32_t* nfp = a.part_nf + slot * a.nparts;
-            auto pulls = [&](uint32_t p, const MbfsPart& P) {
-                const uint32_t x = __ldcg(&nfp[p]);
-                return x > 0 && (double)x > (double)P.n * a.pull_fraction;
-            };
-            // ---- expand, pulling graphs. In-lists of at most kPullChunk
-            // edges: one lane per vertex, scanned whole (4 loads in flight)
-            // until the bits v still needs are covered; longer lists: one
+            for (uint32_t p = tid; p < a.nparts; p += nth) a.part_nf[cnext * a.nparts + p] = 0u;
+            auto pulls = [&](uint32_t p, const MbfsPart& P) { return mode_of(p, P) == kPull; };
+            // a level whose graphs all pull and have no long list is its second
+            // half alone (one barrier instead of two, the same in every block;
+            // a history slot just written out is reused only behind a barrier)
+            const bool halves = S.halves != 0;
+            found += nf;
+            // ---- first half: pulling graphs' lists over kPullChunk edges, one
             // lane per kPullChunk-edge piece from the static piece table,
-            // merged into next[v] with atomicOr. No lane scans more than
-            // kPullChunk edges, so no list sets the level's time.
-            for_each_part_word(a, warp, nwarps, pulls, [&](uint32_t p, const MbfsPart& P, uint32_t wi) {
-                const uint32_t v = wi * 32 + lane;
-                if (v - P.off >= P.n) return;
-                const uint32_t pb = __ldg(&g.csr_ptrs[v]), pe = __ldg(&g.csr_ptrs[v + 1]);
-                if (pe - pb > kPullChunk || pe == pb) return;
-                uint32_t valid[WORDS];
-                rows_mask<WORDS>(group_rows(P, s0, a.group_width), valid);
-                const Bits<WORDS> vis = load_bits<WORDS>(a.visited, v);
-                uint32_t need[WORDS], acc[WORDS];
-                bool any = false;
-#pragma unroll
-                for (int w = 0; w < WORDS; ++w) {
-                    need[w] = ~vis.w[w] & valid[w];
-                    acc[w] = 0u;
-                    any |= need[w] != 0;
-                }
-                if (!any) return;
-                scan_in_list<WORDS>(a, hist_slot<WORDS>(a, level - 1), pb, pe, need, acc);
-                bool got = false;
-                Bits<WORDS> out;
-#pragma unroll
-                for (int w = 0; w < WORDS; ++w) {
-                    out.w[w] = acc[w];
-                    got |= acc[w] != 0;
-                }
-                if (got) store_bits<WORDS>(a.next, v, out);
-            });
+            // merged into next[v] with atomicOr; pushing graphs' tiles. No lane
+            // scans more than kPullChunk edges, so no list sets the level's
+            // time.
             for_each_part_chunks(a, warp, nwarps, pulls, [&](uint32_t p, const MbfsPart& P, uint32_t cb, uint32_t ce) {
                 uint32_t valid[WORDS];
                 rows_mask<WORDS>(group_rows(P, s0, a.group_width), valid);
@@ -500,13 +652,17 @@ __global__ void __launch_bounds__(512, 2) mbfs_persistent_kernel(MbfsArgs a) {
                         if (acc[w]) atomicOr(&a.next[v * WORDS + w], acc[w]);
                 }
             });
-            // ---- expand, pushing graphs: the queued rsets' tiles. Each warp
-            // takes a contiguous range of 32-tile chunks, finds the owner
-            // entry of its first chunk once and walks the queue forward;
-            // entries of pulling graphs are skipped whole.
+            // Pushing graphs: the queued rsets' tiles. Each warp takes a
+            // contiguous range of 32-tile chunks, finds the owner entry of its
+            // first chunk once and walks the queue forward; entries of pulling
+            // graphs are skipped whole.
             const bool single_pulls = !a.parts && pulls(0, a.part0);
-            if (!single_pulls) {
-                const uint64_t qc = ld_relaxed64(&c->aux[slot]);
+            // While under an eighth of the vertices have been found, looking a
+            // row up before marking it filters little (the second half drops
+            // what was visited).
+            const bool look = found > n / 8;
+            if (halves && !single_pulls) {
+                const uint64_t qc = S.queue;
                 const uint32_t E = (uint32_t)(qc >> kQShift), U = (uint32_t)(qc & kQUnitMask);
                 const uint32_t* qr = a.q_rset + slot * a.qreg;
                 const uint32_t* qo = a.q_off + slot * a.qreg;
@@ -592,7 +748,19 @@ __global__ void __launch_bounds__(512, 2) mbfs_persistent_kernel(MbfsArgs a) {
                                 if ((mb >> k) & 1u)
 #pragma unroll
                                     for (int w = 0; w < WORDS; ++w) acc.w[w] |= col[k].w[w];
-                            const Bits<WORDS> vis = load_bits<WORDS>(a.visited, row);
+                            // most slices of a sparse frontier's sets hit no
+                            // frontier column: they need no look at the row
+                            bool hit = false;
+#pragma unroll
+                            for (int w = 0; w < WORDS; ++w) hit |= acc.w[w] != 0;
+                            if (!hit) continue;
+                            Bits<WORDS> vis;
+                            if (look) {
+                                vis = load_bits<WORDS>(a.visited, row);
+                            } else {
+#pragma unroll
+                                for (int w = 0; w < WORDS; ++w) vis.w[w] = 0u;
+                            }
 #pragma unroll
                             for (int w = 0; w < WORDS; ++w) {
                                 const uint32_t add = acc.w[w] & ~vis.w[w];
@@ -603,77 +771,117 @@ __global__ void __launch_bounds__(512, 2) mbfs_persistent_kernel(MbfsArgs a) {
                     }
                 }
             }
-            if (!barrier()) return;
-            // ---- sweep over the active graphs' words (an inactive graph has
-            // an empty frontier and received no next bits)
-            uint32_t cnt = 0;
-            uint32_t* nfn = a.part_nf + (slot ^ 1) * a.nparts;
-            auto active = [&](uint32_t p, const MbfsPart&) { return __ldcg(&nfp[p]) > 0; };
+            if ((halves || written) && !barrier()) return;
+            // ---- second half, over the active graphs' words (an idle graph
+            // has an empty frontier and received no next bits). A pulling
+            // graph's short lists are scanned here, one lane per vertex, until
+            // the bits v still needs are covered; what they find is final, so
+            // it goes straight into `visited` and the history without a trip
+            // through `next`. Long lists and pushing graphs take theirs from
+            // `next`.
+            uint32_t cnt = 0, waiting = 0, total = 0, cntp = 0xFFFFFFFFu;
+            uint32_t* nfn = a.part_nf + cout * a.nparts;
+            uint32_t* qr1 = a.q_rset + (slot ^ 1) * a.qreg;
+            uint32_t* qo1 = a.q_off + (slot ^ 1) * a.qreg;
+            auto active = [&](uint32_t p, const MbfsPart& P) { return mode_of(p, P) != kIdle; };
+            auto count_part = [&]() {  // the vertices found in graph cntp so far
+                const uint32_t sum = __reduce_add_sync(0xFFFFFFFFu, cnt);
+                if (lane == 0 && sum && a.parts) atomicAdd(&nfn[cntp], sum);
+                total += sum;
+                cnt = 0;
+            };
             for_each_part_word(a, warp, nwarps, active, [&](uint32_t p, const MbfsPart& P, uint32_t wi) {
+                if (p != cntp) {
+                    count_part();
+                    cntp = p;
+                }
                 const uint32_t v = wi * 32 + lane;
+                const bool pulling = mode_of(p, P) == kPull;
                 Bits<WORDS> nw;
                 bool any = false;
-                if (v < n) {
-                    const Bits<WORDS> nx = load_bits<WORDS>(a.next, v);
+#pragma unroll
+                for (int w = 0; w < WORDS; ++w) nw.w[w] = 0u;
+                if (v - P.off < P.n) {
                     const Bits<WORDS> vis = load_bits<WORDS>(a.visited, v);
-                    Bits<WORDS> nv;
+                    bool from_next = true;
+                    if (pulling) {
+                        const uint32_t pb = __ldg(&g.csr_ptrs[v]), pe = __ldg(&g.csr_ptrs[v + 1]);
+                        from_next = pe - pb > kPullChunk;
+                        uint32_t need[WORDS], acc[WORDS];
+                        rows_mask<WORDS>(group_rows(P, s0, a.group_width), need);
+                        bool some = false;
 #pragma unroll
-                    for (int w = 0; w < WORDS; ++w) {
-                        nw.w[w] = nx.w[w] & ~vis.w[w];
-                        nv.w[w] = vis.w[w] | nw.w[w];
-                        any |= nw.w[w] != 0;
+                        for (int w = 0; w < WORDS; ++w) {
+                            need[w] &= ~vis.w[w];
+                            acc[w] = 0u;
+                            some |= need[w] != 0;
+                        }
+                        if (!from_next && some && pe > pb) {
+                            scan_in_list<WORDS>(a, hist_slot<WORDS>(a, level - 1), pb, pe, need, acc);
+#pragma unroll
+                            for (int w = 0; w < WORDS; ++w) nw.w[w] = acc[w];
+                        }
                     }
-                    if (any) store_bits<WORDS>(a.visited, v, nv);
-                    // every word of an active graph: the slot held an
-                    // older level
-                    store_bits<WORDS>(hist_slot<WORDS>(a, level), v, nw);
-                    bool nxAny = false;
+                    if (from_next) {
+                        const Bits<WORDS> nx = load_bits<WORDS>(a.next, v);
+                        bool got = false;
 #pragma unroll
-                    for (int w = 0; w < WORDS; ++w) nxAny |= nx.w[w] != 0;
-                    if (nxAny) {
-                        Bits<WORDS> z;
+                        for (int w = 0; w < WORDS; ++w) {
+                            nw.w[w] = nx.w[w] & ~vis.w[w];
+                            got |= nx.w[w] != 0;
+                        }
+                        if (got) {
+                            Bits<WORDS> z;
 #pragma unroll
-                        for (int w = 0; w < WORDS; ++w) z.w[w] = 0u;
-                        store_bits<WORDS>(a.next, v, z);
+                            for (int w = 0; w < WORDS; ++w) z.w[w] = 0u;
+                            store_bits<WORDS>(a.next, v, z);
+                        }
                     }
-                } else {
 #pragma unroll
-                    for (int w = 0; w < WORDS; ++w) nw.w[w] = 0u;
+                    for (int w = 0; w < WORDS; ++w) any |= nw.w[w] != 0;
+                    if (any) {
+                        Bits<WORDS> nv;
+#pragma unroll
+                        for (int w = 0; w < WORDS; ++w) nv.w[w] = vis.w[w] | nw.w[w];
+                        store_bits<WORDS>(a.visited, v, nv);
+                    }
                 }
+                // every word of an active graph: the slot held an older level
+                if (v < n) store_bits<WORDS>(hist_slot<WORDS>(a, level), v, nw);
                 if (lane == 0 && wi * 32 == P.off) a.part_last[p] = level;  // the graph's slot for `level` is valid
                 const uint32_t anyMask = __ballot_sync(0xFFFFFFFFu, any);
                 if (!anyMask) return;
                 cnt += any ? 1u : 0u;
-                if (lane == 0) atomicAdd(&nfn[p], (uint32_t)__popc(anyMask));
                 // queue rsets with new bits (lanes 8j..8j+7 share rset)
-                const uint32_t grpBits = (anyMask >> (lane & ~7u)) & 0xFFu;
-                uint64_t mine = 0;
-                uint32_t r = 0;
-                if ((lane & 7) == 0 && grpBits) {
-                    r = v >> 3;
-                    const uint32_t t = __ldg(&g.rset_tile[r + 1]) - __ldg(&g.rset_tile[r]);
-                    if (t) mine = (1ull << kQShift) | ((t + 31) / 32);
+                uint32_t units = 0;
+                if ((lane & 7) == 0 && ((anyMask >> lane) & 0xFFu)) {
+                    const uint32_t r = v >> 3;
+                    units = (__ldg(&g.rset_tile[r + 1]) - __ldg(&g.rset_tile[r]) + 31) / 32;
                 }
-                const uint64_t incl = warp_inclusive_scan64(mine);
-                const uint64_t tot = __shfl_sync(0xFFFFFFFFu, incl, 31);
-                if (tot) {
-                    uint64_t b0 = 0;
-                    if (lane == 31) b0 = atomicAdd(&c->aux[slot ^ 1], (unsigned long long)tot);
-                    b0 = __shfl_sync(0xFFFFFFFFu, b0, 31);
-                    if (mine) {
-                        const uint64_t ex = b0 + incl - mine;
-                        const uint32_t e = (uint32_t)(ex >> kQShift);
-                        if (e < a.qreg) {
-                            a.q_rset[(slot ^ 1) * a.qreg + e] = r;
-                            a.q_off[(slot ^ 1) * a.qreg + e] = (uint32_t)(ex & kQUnitMask);
-                        } else {
-                            set_error(c, BLEST_ERR_DEVICE_INDEX);
-                        }
-                    }
+                const uint32_t qm = __ballot_sync(0xFFFFFFFFu, units != 0);
+                if (units) {
+                    const uint32_t at = waiting + __popc(qm & ((1u << lane) - 1u));
+                    S.rset[threadIdx.x >> 5][at] = v >> 3;
+                    S.units[threadIdx.x >> 5][at] = units;
+                }
+                waiting += __popc(qm);
+                if (waiting > kQueueBuf - 4) {
+                    flush_rsets(a, S, waiting, &c->aux[cout], qr1, qo1);
+                    waiting = 0;
                 }
             });
-            const uint64_t wc = warp_sum64(cnt);
-            if (lane == 0 && wc) atomicAdd(&c->aux[4 + (slot ^ 1)], (unsigned long long)wc);
+            flush_rsets(a, S, waiting, &c->aux[cout], qr1, qo1);
+            count_part();
+            if (lane == 0) S.cnt[threadIdx.x >> 5] = total;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                uint32_t sum = 0;
+                for (uint32_t i = 0; i < blockDim.x >> 5; ++i) sum += S.cnt[i];
+                if (sum) {
+                    atomicAdd(&c->aux[3 + cout], (unsigned long long)sum);
+                    if (!a.parts) atomicAdd(&nfn[0], sum);
+                }
+            }
             if (tid == 0) c->levels = max(c->levels, level);
             if (!barrier()) return;
         }
@@ -692,7 +900,7 @@ struct MbfsScratch {
     uint32_t* levels = nullptr; // staging for host output
     uint32_t* sources = nullptr;
     uint32_t* queue = nullptr;  // rset queue: 2 slots of entries + 2 slots of offsets
-    uint32_t* part_nf = nullptr;  // per-graph frontier counts, 2 slots
+    uint32_t* part_nf = nullptr;  // per-graph frontier counts, 3 slots
     uint32_t* part_last = nullptr;  // per-graph last level with a valid history slot
     uint32_t* rows = nullptr;  // per-source output pointers (2 words each)
     size_t state_words = 0, levels_words = 0, sources_cap = 0, queue_words = 0, part_nf_cap = 0,
@@ -740,7 +948,7 @@ void prepare_words(const blest_graph* g, blest::Workspace& w, MbfsScratch& sc, c
     ensure(sc.queue, sc.queue_words, 4ull * a.qreg);
     a.q_rset = sc.queue;
     a.q_off = sc.queue + 2ull * a.qreg;
-    ensure(sc.part_nf, sc.part_nf_cap, 2ull * nparts);
+    ensure(sc.part_nf, sc.part_nf_cap, 3ull * nparts);
     a.part_nf = sc.part_nf;
     a.trace = p.trace ? w.trace : nullptr;
     a.ctr = w.counters;
@@ -797,7 +1005,7 @@ void mbfs_reserve(Workspace& w, uint32_t n, uint32_t words) {
     ensure(sc.state, sc.state_words, mbfs_state_words(n, words));
     ensure(sc.sources, sc.sources_cap, 128);
     ensure(sc.queue, sc.queue_words, 4ull * mbfs_queue_slot((n + 7) / 8, 32u * words));
-    ensure(sc.part_nf, sc.part_nf_cap, 2);
+    ensure(sc.part_nf, sc.part_nf_cap, 3);
     ensure(sc.part_last, sc.part_last_cap, 1);
 }
 
@@ -902,7 +1110,7 @@ void join_graphs(const std::vector<const blest_graph*>& gs, const std::vector<ui
     uint32_t* masks = plan_alloc<uint32_t>(u, T);
     uint32_t* rt = plan_alloc<uint32_t>(u, (size_t)R + 1);
     uint32_t* cp = plan_alloc<uint32_t>(u, (size_t)N + 1);
-    uint32_t* ci = plan_alloc<uint32_t>(u, E);
+    uint32_t* ci = plan_alloc<uint32_t>(u, E + 8);  // whole quads past the end
     uint32_t* hin = plan_alloc<uint32_t>(u, (size_t)N / 32 + 4);
     uint4* pieces = plan_alloc<uint4>(u, C);
     std::vector<JoinSeg> segs;
