@@ -148,6 +148,9 @@ void workspace_alloc(const blest_graph* g, Workspace& w) {
     alloc((void**)&w.q_rset, 4ull * w.qcap);
     alloc((void**)&w.q_off, 4ull * w.qcap);
     alloc((void**)&w.counters, sizeof(dev::RunCounters));
+    alloc((void**)&w.list_counters, sizeof(dev::RunCounters));
+    BLEST_CUDA(cudaMemset(w.list_counters, 0, sizeof(dev::RunCounters)));
+    BLEST_CUDA(cudaStreamSynchronize(nullptr));
     alloc((void**)&w.levels, 4ull * n);
     alloc((void**)&w.parents, 4ull * n);
     alloc((void**)&w.cc_parent, 8ull * n);
@@ -172,6 +175,7 @@ void workspace_free(Workspace& w) {
     cudaFree(w.q_rset);
     cudaFree(w.q_off);
     cudaFree(w.counters);
+    cudaFree(w.list_counters);
     cudaFree(w.levels);
     cudaFree(w.parents);
     cudaFree(w.cc_parent);
@@ -270,19 +274,23 @@ void finish_one(blest_workspace* ws, blest_bfs_stats* st) {
         // slot; either way the slot's last copy is then done
         BLEST_CUDA(cudaEventSynchronize(ws->ev_copy[slot]));
         ws->slot_busy[slot] = false;
-    } else if (slot < 0 && seq + 1 == ws->issued) {
+    } else if (slot == blest::kCallStream && seq + 1 == ws->issued) {
         // the last call issued: the stream's completion is this call's
         BLEST_CUDA(cudaStreamSynchronize(ws->stream));
     } else if (slot < 0) {
-        // Wait for this call's record only (later calls keep running): its
-        // kernel writes seq last, after a system-scope fence. If the stream
-        // has drained and the record is still missing, the call failed.
+        // Wait for this call's record (later calls keep running): its kernel
+        // writes seq last, after a system-scope fence, which the host sees
+        // several microseconds before the stream reports completion. If the
+        // stream has drained and the record is still missing, the call failed.
         const volatile unsigned long long* vs = &w.records[seq % blest::kRecordRing].seq;
-        for (uint32_t spin = 0; *vs != seq; ++spin) {
+        const auto start = std::chrono::steady_clock::now();
+        for (uint32_t spin = 1; *vs != seq; ++spin) {
+            if (spin % 16384) continue;  // tens of microseconds between two looks at the stream
             const cudaError_t q = cudaStreamQuery(ws->stream);
             if (q == cudaSuccess) break;
             if (q != cudaErrorNotReady) BLEST_CUDA(q);
-            if (spin > 64) std::this_thread::sleep_for(std::chrono::microseconds(20));
+            if (std::chrono::steady_clock::now() - start > std::chrono::milliseconds(2))
+                std::this_thread::sleep_for(std::chrono::microseconds(20));
         }
         std::atomic_thread_fence(std::memory_order_acquire);
     }
@@ -623,7 +631,10 @@ int blest_bfs_ws(blest_workspace* ws, uint32_t source, uint32_t* levels_out, uin
         uint32_t* hp = slot ? w.parents_b : w.parents;
         uint32_t* dl = out_mem == BLEST_MEM_DEVICE ? levels_out : hl;
         uint32_t* dp = parents_out ? (out_mem == BLEST_MEM_DEVICE ? parents_out : hp) : nullptr;
-        w.call_slot[seq % blest::kRecordRing] = (int8_t)(pipelined ? slot : -1);
+        // the kernel over tiles leaves its record before its last block has left
+        const bool polled = out_mem == BLEST_MEM_DEVICE && g->d.out_ptrs && p.slice_test != BLEST_TEST_B1_MMA;
+        w.call_slot[seq % blest::kRecordRing] =
+            pipelined ? (int8_t)slot : (polled ? blest::kCallPolled : blest::kCallStream);
         blest::launch_bfs(g, w, source, dl, dp, p, s, seq);
         ws->issued = seq + 1;
         ws->stream = s;
@@ -667,12 +678,17 @@ int blest_workspace_trace(blest_workspace* ws, blest_level_trace* out, uint32_t 
     return guarded([&] {
         blest::require(ws && out && count, "null argument");
         BLEST_CUDA(cudaSetDevice(ws->g->device));
-        // BFS: one record per level + the end record; MBFS counts its own.
-        // The counters of the last run are still on the device.
-        blest::dev::RunCounters c;
-        BLEST_CUDA(cudaMemcpy(&c, ws->w.counters, sizeof(c), cudaMemcpyDeviceToHost));
-        const uint32_t recs = c.trace_records;
-        const uint32_t levels = recs ? recs : c.levels + 1;
+        // BFS: one record per level + the end record; MBFS counts its own. The
+        // counters of the last run are still on the device, or (BFS over
+        // lists) its levels in its record.
+        uint32_t levels = 0;
+        if (ws->w.trace_seq >= 0) {
+            levels = ws->w.records[ws->w.trace_seq % blest::kRecordRing].levels + 1;
+        } else {
+            blest::dev::RunCounters c;
+            BLEST_CUDA(cudaMemcpy(&c, ws->w.counters, sizeof(c), cudaMemcpyDeviceToHost));
+            levels = c.trace_records ? c.trace_records : c.levels + 1;
+        }
         const uint32_t k = std::min<uint32_t>(std::min<uint32_t>(levels, max), BLEST_TRACE_CAPACITY);
         BLEST_CUDA(cudaMemcpy(out, ws->w.trace, sizeof(blest_level_trace) * k, cudaMemcpyDeviceToHost));
         *count = k;

@@ -923,7 +923,12 @@ template <bool ALIGNED, bool MMA, bool PARENTS>
 __global__ void __launch_bounds__(512, 2) bfs_persistent_kernel(BfsArgs a) {
     const uint64_t t0 = global_ns();
     bfs_run<ALIGNED, MMA, PARENTS>(a);
-    write_record(a, t0);
+    // thread 0 of block 0 wrote the counts itself, and an error recorded by any
+    // block was visible to it at the barrier that ended its run
+    if (a.record && blockIdx.x == 0 && threadIdx.x == 0) {
+        fill_record(a.record, a, t0);
+        publish_record(a.record, a.seq);
+    }
 }
 
 }  // namespace dev
@@ -996,8 +1001,11 @@ void launch_bfs(const blest_graph* g, Workspace& w, uint32_t src, uint32_t* leve
     const int threads = p.threads_per_block > 0 ? p.threads_per_block : 512;
     if (threads % 32 || threads > 512) throw Error(BLEST_ERR_INVALID_ARG, "threads_per_block must be a multiple of 32, <= 512");
     const bool mma = p.slice_test == BLEST_TEST_B1_MMA;
+    w.trace_seq = -1;
     if (!mma && g->d.out_ptrs) {
         a.pieces = w.pieces;
+        a.ctr = w.list_counters;
+        w.trace_seq = (int64_t)seq;
         launch_bfs_lists(g, a, p.blocks_per_sm, threads, w.grid_blocks, s);
         return;
     }

@@ -54,13 +54,10 @@ constexpr uint32_t kPullUnroll = 4;
 // Neighbours per piece of a heavy (very long) in-neighbour list.
 constexpr uint32_t kHeavyChunk = 256;
 
-// The run's record, by the kernel's last thread (thread 0 of block 0 wrote the
-// counts itself, and an error recorded by any block was visible to it at the
-// barrier that ended its run).
-__device__ __forceinline__ void write_record(const BfsArgs& a, uint64_t start_ns) {
-    if (!a.record || blockIdx.x != 0 || threadIdx.x != 0) return;
+// The run's record but its seq, which the host polls and which must become
+// visible after the rest.
+__device__ __forceinline__ void fill_record(RunRecord* r, const BfsArgs& a, uint64_t start_ns) {
     const RunCounters* c = a.ctr;
-    RunRecord* r = a.record;
     r->start_ns = start_ns;
     r->end_ns = global_ns();
     r->error = ld_relaxed(&c->error);
@@ -70,9 +67,11 @@ __device__ __forceinline__ void write_record(const BfsArgs& a, uint64_t start_ns
     r->push_levels = c->push_levels;
     r->pull_levels = c->pull_levels;
     r->source = a.src;
-    // the host polls seq: it must become visible after the rest
+}
+
+__device__ __forceinline__ void publish_record(RunRecord* r, uint64_t seq) {
     __threadfence_system();
-    *(volatile unsigned long long*)&r->seq = a.seq;
+    *(volatile unsigned long long*)&r->seq = seq;
 }
 
 }  // namespace dev

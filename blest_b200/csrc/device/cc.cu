@@ -582,6 +582,7 @@ void launch_cc_union(const blest_graph* g, Workspace& w, uint32_t* labels, cudaS
     BLEST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxBlocks, dev::cc_union_kernel, threads, 0));
     if (maxBlocks < 1) throw Error(BLEST_ERR_CUDA, "CC kernel cannot be resident");
     // no more blocks than vertices / threads: every block costs the barriers
+    w.trace_seq = -1;
     const int grid = std::min(cooperative_grid(maxBlocks, g->sm_count, w.grid_blocks),
                               (int)((g->d.n + threads - 1) / threads));
     BLEST_CUDA(cudaMemsetAsync(w.counters, 0, sizeof(dev::RunCounters), s));

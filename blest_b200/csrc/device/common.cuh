@@ -100,7 +100,9 @@ struct RunCounters {
     // Grid barrier: monotone arrival count (bits 0-62) + error flag (bit 63),
     // alone on its 128-byte line.
     alignas(128) unsigned long long arrive;
-    unsigned long long pad_arrive[15];
+    unsigned long long exits;     // BFS over lists: blocks that have left
+    unsigned long long start_ns;  // and its block 0's start
+    unsigned long long pad_arrive[13];
 };
 
 // Outcome of one single-source BFS launch, written by the kernel itself as
@@ -175,8 +177,11 @@ __device__ __forceinline__ void set_error(RunCounters* c, uint32_t code) {
 // one timed-out block ends the wait of all the others. Returns the final
 // counter value (bit 63 = error recorded).
 __device__ __forceinline__ uint64_t barrier_arrive_wait(RunCounters* c, uint64_t expected, uint64_t timeout_ns) {
-    __threadfence();
-    uint64_t v = atomicAdd(&c->arrive, 1ull);
+    // Release and acquire ride on the arrival itself and on the polls: a fence
+    // on either side (__threadfence is a sequentially consistent one) costs
+    // every barrier hundreds of nanoseconds.
+    uint64_t v;
+    asm volatile("atom.add.acq_rel.gpu.global.u64 %0, [%1], 1;" : "=l"(v) : "l"(&c->arrive) : "memory");
     const uint64_t target = ((v & ~kArriveError) / expected + 1) * expected;
     ++v;
     if ((v & ~kArriveError) < target && !(v & kArriveError)) {
@@ -191,7 +196,6 @@ __device__ __forceinline__ uint64_t barrier_arrive_wait(RunCounters* c, uint64_t
             if (spins > 256) __nanosleep(20);
         }
     }
-    __threadfence();
     return v;
 }
 

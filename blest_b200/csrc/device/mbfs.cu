@@ -951,6 +951,7 @@ void prepare_words(const blest_graph* g, blest::Workspace& w, MbfsScratch& sc, c
     ensure(sc.part_nf, sc.part_nf_cap, 3ull * nparts);
     a.part_nf = sc.part_nf;
     a.trace = p.trace ? w.trace : nullptr;
+    w.trace_seq = -1;
     a.ctr = w.counters;
     a.group_width = 32 * WORDS;
     a.pull_fraction = p.pull_fraction > 0 ? (float)p.pull_fraction : 1.0f / 64.0f;

@@ -33,6 +33,8 @@ struct Workspace {
     uint32_t* q_rset = nullptr;
     uint32_t* q_off = nullptr;
     dev::RunCounters* counters = nullptr;
+    dev::RunCounters* list_counters = nullptr;  // BFS over lists: zero between runs
+    int64_t trace_seq = -1;                     // BFS over lists: the last run's call number (-1: another kernel ran)
     uint32_t* levels = nullptr;   // internal output buffers (host-output calls)
     uint32_t* parents = nullptr;
     uint32_t* cc_parent = nullptr;  // CC: union-find parents and kept edges, n words each
@@ -51,7 +53,8 @@ struct Workspace {
     // kRecordRing: mapped pinned host memory that the kernel writes
     // directly, so reading a finished call's record needs no copy.
     dev::RunRecord* records = nullptr;
-    // Pipelined slot (0/1) of each call, or -1 (same ring positions).
+    // Of each call (same ring positions): its pipelined slot (0/1), kCallPolled
+    // (done when its record is there) or kCallStream (when its stream is).
     int8_t* call_slot = nullptr;
     // Second level/parent buffers of the pipelined host-output mode (the
     // first pair is `levels`/`parents`), allocated on first use.
@@ -59,6 +62,8 @@ struct Workspace {
     uint32_t* parents_b = nullptr;
     uint64_t bytes = 0;
 };
+
+constexpr int8_t kCallPolled = -1, kCallStream = -2;
 
 // Asynchronous BFS calls whose outcome a workspace keeps until
 // blest_workspace_sync reads it.

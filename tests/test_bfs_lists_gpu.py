@@ -92,3 +92,50 @@ def test_directed_out_hub(gpu):
 def test_uniform_dense_levels(gpu):
     """A level whose edges outnumber n / 4 (marked first, swept after)."""
     check(Csc.er(100_003, 1_600_000, seed=3), [0, 777])
+
+
+def test_pull_then_push_queues_its_finds(gpu):
+    """A dense core (pulled) with tails hanging off it: the pull level that
+    finds the tails' ends queues them for the push levels that follow, a few
+    and several thousand (more than a block's buffer), with and without the
+    grid's cap."""
+    for tails, spread in ((5, 1), (3000, 1), (9000, 2)):
+        core = Csc.er(20_000, 400_000, seed=tails)
+        src = np.repeat(np.arange(core.n), core.degrees()).astype(np.int64)
+        dst = core.rows.astype(np.int64)
+        at = core.n + np.arange(tails * 3).reshape(tails, 3)
+        base = (np.arange(tails) * spread) % core.n
+        a = np.concatenate([base, at[:, 0], at[:, 1]])
+        b = np.concatenate([at[:, 0], at[:, 1], at[:, 2]])
+        csc = Csc.from_edges(core.n + tails * 3, np.concatenate([src, a, b]), np.concatenate([dst, b, a]))
+        check(csc, [0, csc.n - 1])
+        check(csc, [7], threads_per_block=32, blocks_per_sm=1)
+
+
+def test_calls_back_to_back_and_between_other_kernels(gpu):
+    """The counters that one run leaves clean serve the next, whatever ran in
+    between on the workspace and whichever stream the next call takes."""
+    import torch
+
+    from blest_b200 import Workspace
+    csc = Csc.rmat(12, 8, seed=3, permute_seed=4)
+    g = Graph(Bvss.build(csc), csc.transpose())
+    ws = Workspace(g)
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    outs = [torch.empty(csc.n, dtype=torch.int32, device="cuda") for _ in range(12)]
+    want = [O.bfs_csc(csc.n, csc.col_ptrs, csc.rows, s) for s in range(12)]
+    labels = torch.empty(csc.n, dtype=torch.int32, device="cuda")
+    for rep in range(20):
+        for i, out in enumerate(outs):
+            out.fill_(7)
+            torch.cuda.synchronize()
+            ws.bfs_async(i, out.data_ptr(), streams[i % 3].cuda_stream)
+            st = ws.sync()
+            assert st.source_vertex == i and st.no_visited == int((want[i] != O.UNREACHED).sum())
+            if i % 4 == 1:
+                ws.cc(labels.data_ptr(), stream=streams[0].cuda_stream)
+            if i % 4 == 2:
+                ws.mbfs_rows([0, i], [outs[0].data_ptr(), labels.data_ptr()], stream=streams[1].cuda_stream)
+            if i % 4 == 3:
+                g.bfs(i, params=bfs_params("auto", "mma"))
+            np.testing.assert_array_equal(out.cpu().numpy().view(np.uint32), want[i])
