@@ -149,7 +149,9 @@ void workspace_alloc(const blest_graph* g, Workspace& w) {
     alloc((void**)&w.q_off, 4ull * w.qcap);
     alloc((void**)&w.counters, sizeof(dev::RunCounters));
     alloc((void**)&w.list_counters, sizeof(dev::RunCounters));
+    alloc((void**)&w.cc_counters, sizeof(dev::RunCounters));
     BLEST_CUDA(cudaMemset(w.list_counters, 0, sizeof(dev::RunCounters)));
+    BLEST_CUDA(cudaMemset(w.cc_counters, 0, sizeof(dev::RunCounters)));
     BLEST_CUDA(cudaStreamSynchronize(nullptr));
     alloc((void**)&w.levels, 4ull * n);
     alloc((void**)&w.parents, 4ull * n);
@@ -162,7 +164,9 @@ void workspace_alloc(const blest_graph* g, Workspace& w) {
     alloc((void**)&w.heavy, sizeof(uint4) * w.heavy_cap);
     BLEST_CUDA(cudaMallocHost((void**)&w.host_counters, sizeof(dev::RunCounters)));
     BLEST_CUDA(cudaHostAlloc((void**)&w.records, sizeof(dev::RunRecord) * kRecordRing, cudaHostAllocMapped));
+    BLEST_CUDA(cudaHostAlloc((void**)&w.cc_record, sizeof(dev::CcRecord), cudaHostAllocMapped));
     // no slot may look like a finished call before its kernel wrote it
+    std::memset((void*)w.cc_record, 0xFF, sizeof(dev::CcRecord));
     std::memset((void*)w.records, 0xFF, sizeof(dev::RunRecord) * kRecordRing);
     w.call_slot = new int8_t[kRecordRing];
     BLEST_CUDA(cudaEventCreate(&w.ev_start));
@@ -176,6 +180,7 @@ void workspace_free(Workspace& w) {
     cudaFree(w.q_off);
     cudaFree(w.counters);
     cudaFree(w.list_counters);
+    cudaFree(w.cc_counters);
     cudaFree(w.levels);
     cudaFree(w.parents);
     cudaFree(w.cc_parent);
@@ -185,6 +190,7 @@ void workspace_free(Workspace& w) {
     cudaFree(w.heavy);
     mbfs_scratch_free(w.mbfs);
     if (w.records) cudaFreeHost(w.records);
+    if (w.cc_record) cudaFreeHost(w.cc_record);
     delete[] w.call_slot;
     cudaFree(w.levels_b);
     cudaFree(w.parents_b);
@@ -253,6 +259,24 @@ void release_pipeline(blest_workspace* ws) {
     }
 }
 
+// Wait until a record carries `seq`: its kernel writes that last, after a
+// system-scope fence, which the host sees several microseconds before the
+// stream reports completion. Returns too when the stream has drained without
+// it (the call failed: the caller finds the record missing).
+void await_record(const unsigned long long* at, uint64_t seq, cudaStream_t stream) {
+    const volatile unsigned long long* vs = at;
+    const auto start = std::chrono::steady_clock::now();
+    for (uint32_t spin = 1; *vs != seq; ++spin) {
+        if (spin % 16384) continue;  // tens of microseconds between two looks at the stream
+        const cudaError_t q = cudaStreamQuery(stream);
+        if (q == cudaSuccess) break;
+        if (q != cudaErrorNotReady) BLEST_CUDA(q);
+        if (std::chrono::steady_clock::now() - start > std::chrono::milliseconds(2))
+            std::this_thread::sleep_for(std::chrono::microseconds(20));
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+}
+
 // Settle the oldest BFS call issued on `ws` and not yet checked: wait
 // until it is done (its host copy, for a pipelined call; the stream
 // otherwise), read its record and report its failure. `st` gets its
@@ -278,21 +302,8 @@ void finish_one(blest_workspace* ws, blest_bfs_stats* st) {
         // the last call issued: the stream's completion is this call's
         BLEST_CUDA(cudaStreamSynchronize(ws->stream));
     } else if (slot < 0) {
-        // Wait for this call's record (later calls keep running): its kernel
-        // writes seq last, after a system-scope fence, which the host sees
-        // several microseconds before the stream reports completion. If the
-        // stream has drained and the record is still missing, the call failed.
-        const volatile unsigned long long* vs = &w.records[seq % blest::kRecordRing].seq;
-        const auto start = std::chrono::steady_clock::now();
-        for (uint32_t spin = 1; *vs != seq; ++spin) {
-            if (spin % 16384) continue;  // tens of microseconds between two looks at the stream
-            const cudaError_t q = cudaStreamQuery(ws->stream);
-            if (q == cudaSuccess) break;
-            if (q != cudaErrorNotReady) BLEST_CUDA(q);
-            if (std::chrono::steady_clock::now() - start > std::chrono::milliseconds(2))
-                std::this_thread::sleep_for(std::chrono::microseconds(20));
-        }
-        std::atomic_thread_fence(std::memory_order_acquire);
+        // this call's record (later calls keep running)
+        await_record(&w.records[seq % blest::kRecordRing].seq, seq, ws->stream);
     }
     const blest::dev::RunRecord& r = w.records[seq % blest::kRecordRing];
     if (r.seq != seq) throw blest::Error(BLEST_ERR_CUDA, "BFS call " + std::to_string(seq) + " left no record");
@@ -720,6 +731,25 @@ int blest_cc_ws(blest_workspace* ws, uint32_t* labels_out, int out_mem, void* st
         cudaStream_t s = stream ? (cudaStream_t)stream : (ws->stream ? ws->stream : g->stream);
         blest::Workspace& w = ws->w;
         uint32_t* dl = out_mem == BLEST_MEM_DEVICE ? labels_out : w.levels;
+        if (g->symmetric) {
+            const uint64_t seq = w.cc_calls++;
+            blest::launch_cc_union(g, w, dl, s, seq);
+            if (out_mem == BLEST_MEM_HOST) {
+                BLEST_CUDA(cudaMemcpyAsync(labels_out, dl, 4ull * g->d.n, cudaMemcpyDeviceToHost, s));
+                BLEST_CUDA(cudaStreamSynchronize(s));
+            } else {
+                await_record(&w.cc_record->seq, seq, s);
+            }
+            const blest::dev::CcRecord& r = *w.cc_record;
+            if (r.seq != seq) throw blest::Error(BLEST_ERR_CUDA, "CC call left no record");
+            if (r.error) throw blest::Error((int)r.error, "device grid barrier timed out");
+            if (stats) {
+                stats->time = (double)(r.end_ns - r.start_ns) * 1e-9;
+                stats->no_components = (uint32_t)r.components;
+                stats->iterations = r.iterations;
+            }
+            return;
+        }
         BLEST_CUDA(cudaEventRecord(w.ev_start, s));
         blest::launch_cc(g, w, dl, s);
         BLEST_CUDA(cudaEventRecord(w.ev_stop, s));

@@ -1188,14 +1188,9 @@ __global__ void __launch_bounds__(512, 2) bfs_lists_kernel(BfsArgs a) {
     // The last block to leave writes the record and zeroes the counters, so
     // that the next run needs no memset before it and a host that sees the
     // record knows that nothing of this run is still to come.
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    unsigned long long left;
-    asm volatile("atom.add.acq_rel.gpu.global.u64 %0, [%1], 1;" : "=l"(left) : "l"(&c->exits) : "memory");
-    if (left + 1 != gridDim.x) return;
+    if (!last_block_out(c)) return;
     if (a.record) fill_record(a.record, a, ld_relaxed64(&c->start_ns));
-    unsigned long long* words = reinterpret_cast<unsigned long long*>(c);
-    for (uint32_t i = 0; i < sizeof(RunCounters) / 8; ++i) words[i] = 0ull;
+    zero_counters(c);
     if (a.record) publish_record(a.record, a.seq);
 }
 

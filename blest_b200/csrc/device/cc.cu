@@ -18,6 +18,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <map>
+#include <mutex>
 
 #include "../host/common.hpp"
 #include "common.cuh"
@@ -306,7 +308,9 @@ struct CcUnionArgs {
     uint32_t* labels;
     uint32_t* parent;  // n words of scratch
     uint32_t* kept;    // n words of scratch: the sampled edge not used in A, v itself when it is settled
-    RunCounters* ctr;
+    RunCounters* ctr;  // zero between runs (the last block out clears them)
+    CcRecord* record;  // mapped host memory
+    unsigned long long seq;
 };
 
 // Position of v in the trees' order, given its degree: degree descending,
@@ -374,7 +378,7 @@ constexpr uint32_t kCcRounds = 12;  // most rounds of R (one counter each in Run
 constexpr uint32_t kCcSamples = 256;
 static_assert(kCcRounds <= 12, "RunCounters::lvl has 12 counters");
 
-__global__ void __launch_bounds__(512, 3) cc_union_kernel(CcUnionArgs a) {
+__device__ __forceinline__ void cc_union_run(const CcUnionArgs& a) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t nth = gridDim.x * blockDim.x;
@@ -566,37 +570,54 @@ __global__ void __launch_bounds__(512, 3) cc_union_kernel(CcUnionArgs a) {
     if (tid == 0) c->iterations = g.nnz ? 2 : 0;  // two phases read the edges (A and D)
 }
 
+__global__ void __launch_bounds__(512, 3) cc_union_kernel(CcUnionArgs a) {
+    RunCounters* c = a.ctr;
+    if (blockIdx.x == 0 && threadIdx.x == 0) c->start_ns = global_ns();
+    cc_union_run(a);
+    if (!last_block_out(c)) return;
+    CcRecord* r = a.record;
+    r->start_ns = ld_relaxed64(&c->start_ns);
+    r->end_ns = global_ns();
+    r->components = ld_relaxed64(&c->discovered);
+    r->error = ld_relaxed(&c->error);
+    r->iterations = ld_relaxed(&c->iterations);
+    zero_counters(c);
+    __threadfence_system();
+    *(volatile unsigned long long*)&r->seq = a.seq;
+}
+
 }  // namespace dev
 
-namespace {
-
-void launch_cc_union(const blest_graph* g, Workspace& w, uint32_t* labels, cudaStream_t s) {
+void launch_cc_union(const blest_graph* g, Workspace& w, uint32_t* labels, cudaStream_t s, uint64_t seq) {
     dev::CcUnionArgs a{};
     a.g = g->d;
     a.labels = labels;
     a.parent = w.cc_parent;
     a.kept = w.cc_parent + g->d.n;
-    a.ctr = w.counters;
+    a.ctr = w.cc_counters;
+    a.record = w.cc_record;
+    a.seq = seq;
     const int threads = 512;
+    // asked once per device (the query costs microseconds)
+    static std::mutex mu;
+    static std::map<int, int> occupancy;
     int maxBlocks = 0;
-    BLEST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxBlocks, dev::cc_union_kernel, threads, 0));
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        int& known = occupancy[g->device];
+        if (!known)
+            BLEST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&known, dev::cc_union_kernel, threads, 0));
+        maxBlocks = known;
+    }
     if (maxBlocks < 1) throw Error(BLEST_ERR_CUDA, "CC kernel cannot be resident");
     // no more blocks than vertices / threads: every block costs the barriers
-    w.trace_seq = -1;
     const int grid = std::min(cooperative_grid(maxBlocks, g->sm_count, w.grid_blocks),
                               (int)((g->d.n + threads - 1) / threads));
-    BLEST_CUDA(cudaMemsetAsync(w.counters, 0, sizeof(dev::RunCounters), s));
     void* kargs[] = {(void*)&a};
     BLEST_CUDA(cudaLaunchCooperativeKernel((void*)dev::cc_union_kernel, grid, threads, kargs, 0, s));
 }
 
-}  // namespace
-
 void launch_cc(const blest_graph* g, Workspace& w, uint32_t* labels, cudaStream_t s) {
-    if (g->symmetric) {
-        launch_cc_union(g, w, labels, s);
-        return;
-    }
     dev::CcArgs a{};
     a.g = g->d;
     a.labels = labels;
@@ -615,6 +636,7 @@ void launch_cc(const blest_graph* g, Workspace& w, uint32_t* labels, cudaStream_
     BLEST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxBlocks, dev::cc_persistent_kernel, threads, 0));
     if (maxBlocks < 1) throw Error(BLEST_ERR_CUDA, "CC kernel cannot be resident");
     const int grid = cooperative_grid(maxBlocks, g->sm_count, w.grid_blocks);
+    w.trace_seq = -1;
     BLEST_CUDA(cudaMemsetAsync(w.counters, 0, sizeof(dev::RunCounters), s));
     dev::cc_init_kernel<<<g->sm_count * 4, 512, 0, s>>>(a);
     BLEST_CUDA(cudaGetLastError());

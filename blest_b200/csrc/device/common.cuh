@@ -100,8 +100,8 @@ struct RunCounters {
     // Grid barrier: monotone arrival count (bits 0-62) + error flag (bit 63),
     // alone on its 128-byte line.
     alignas(128) unsigned long long arrive;
-    unsigned long long exits;     // BFS over lists: blocks that have left
-    unsigned long long start_ns;  // and its block 0's start
+    unsigned long long exits;     // BFS over lists, union-find: blocks that have left
+    unsigned long long start_ns;  // and block 0's start
     unsigned long long pad_arrive[13];
 };
 
@@ -123,6 +123,15 @@ struct RunRecord {
     unsigned int pad;
 };
 static_assert(sizeof(RunRecord) == 64, "RunRecord is one 64-byte slot");
+
+// Outcome of one union-find run, written by its last block into mapped host
+// memory (seq last).
+struct CcRecord {
+    unsigned long long seq;
+    unsigned long long start_ns, end_ns;
+    unsigned long long components;
+    unsigned int error, iterations;
+};
 
 __device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
     uint32_t v;
@@ -215,6 +224,21 @@ __device__ __forceinline__ bool grid_barrier(RunCounters* c, uint64_t expected, 
 }
 
 __device__ __forceinline__ bool grid_barrier(RunCounters* c) { return grid_barrier(c, gridDim.x, kBarrierTimeoutNs); }
+
+// True in one thread of the grid: thread 0 of the block that leaves last (every
+// block calls this once, as its last act; all threads).
+__device__ __forceinline__ bool last_block_out(RunCounters* c) {
+    __syncthreads();
+    if (threadIdx.x != 0) return false;
+    unsigned long long left;
+    asm volatile("atom.add.acq_rel.gpu.global.u64 %0, [%1], 1;" : "=l"(left) : "l"(&c->exits) : "memory");
+    return left + 1 == gridDim.x;
+}
+
+__device__ __forceinline__ void zero_counters(RunCounters* c) {
+    unsigned long long* words = reinterpret_cast<unsigned long long*>(c);
+    for (uint32_t i = 0; i < sizeof(RunCounters) / 8; ++i) words[i] = 0ull;
+}
 
 // Warp-inclusive scan of a 64-bit value.
 __device__ __forceinline__ uint64_t warp_inclusive_scan64(uint64_t v) {

@@ -34,6 +34,9 @@ struct Workspace {
     uint32_t* q_off = nullptr;
     dev::RunCounters* counters = nullptr;
     dev::RunCounters* list_counters = nullptr;  // BFS over lists: zero between runs
+    dev::RunCounters* cc_counters = nullptr;    // union-find: the same
+    dev::CcRecord* cc_record = nullptr;         // union-find: the last run's outcome (mapped host memory)
+    uint64_t cc_calls = 0;                      // runs issued
     int64_t trace_seq = -1;                     // BFS over lists: the last run's call number (-1: another kernel ran)
     uint32_t* levels = nullptr;   // internal output buffers (host-output calls)
     uint32_t* parents = nullptr;
@@ -129,6 +132,9 @@ void launch_bfs(const blest_graph* g, Workspace& w, uint32_t src, uint32_t* leve
 void launch_bfs_lists(const blest_graph* g, const dev::BfsArgs& args, int blocks_per_sm, int threads,
                       uint32_t grid_cap, cudaStream_t s);
 void launch_cc(const blest_graph* g, Workspace& w, uint32_t* labels, cudaStream_t s);
+// Symmetric graphs: run number `seq`, whose outcome the kernel writes to
+// w.cc_record.
+void launch_cc_union(const blest_graph* g, Workspace& w, uint32_t* labels, cudaStream_t s, uint64_t seq);
 
 int device_sm_count(int device);
 

@@ -71,3 +71,30 @@ def test_one_missing_reverse_edge(gpu):
     d = Csc.from_edges(csc.n, src[keep], dst[keep])
     lab, _ = Graph(Bvss.build(d), d.transpose()).cc()
     np.testing.assert_array_equal(lab, O.cc_csc(d.n, d.col_ptrs, d.rows))
+
+
+def test_calls_back_to_back(gpu):
+    """Runs leave their counters clean for the next, on any stream, with BFS
+    and multi-source runs in between and with results on either side."""
+    import torch
+
+    from blest_b200 import Workspace
+    csc = Csc.rmat(11, 4, seed=6, permute_seed=2)
+    want = O.cc_csc(csc.n, csc.col_ptrs, csc.rows)
+    g = Graph.from_csc(csc)
+    ws = Workspace(g)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    out = torch.empty(csc.n, dtype=torch.int32, device="cuda")
+    lev = torch.empty(csc.n, dtype=torch.int32, device="cuda")
+    for i in range(40):
+        out.fill_(-5)
+        torch.cuda.synchronize()
+        st = ws.cc(out.data_ptr(), stream=streams[i % 2].cuda_stream)
+        assert st.no_components == np.unique(want).size and st.time > 0
+        np.testing.assert_array_equal(out.cpu().numpy().view(np.uint32), want)
+        if i % 3 == 0:
+            ws.bfs_async(i, lev.data_ptr(), streams[1].cuda_stream)
+            ws.sync()
+        if i % 3 == 1:
+            ws.mbfs_rows([i], [lev.data_ptr()], stream=streams[0].cuda_stream)
+        np.testing.assert_array_equal(g.cc()[0], want)
