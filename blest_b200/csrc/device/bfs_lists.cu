@@ -236,29 +236,48 @@ __device__ __forceinline__ Flushed flush(const BfsArgs& a, BlockState& B, const 
     __syncthreads();
     const uint32_t m = min(B.win_cnt, B.win_end);
     const bool spilled = B.win_end != kWinners;
-    // A one-block level of few discoveries (m is the same in every thread):
-    // one warp does it all, the discoveries' own degrees are the counts.
-    if (solo && m <= 32 && a.g.out_ptrs == a.g.csr_ptrs) {
+    // Few discoveries (m is the same in every thread), as in most levels: one
+    // warp does it all, and the discoveries' own degrees are the counts (a
+    // block-wide scan costs two more barriers, a microsecond of a 6 us level).
+    if (m <= 32 && !spilled && a.g.out_ptrs == a.g.csr_ptrs) {
+        Flushed F{0, m, 0, false};
         if (w == 0) {
             const uint32_t d = lane < m ? B.win_d[lane] : 0u, b = lane < m ? B.win_b[lane] : 0u;
-            const uint32_t v = lane < m ? B.win_v[lane] : 0u, np = pieces_of(d);
-            const uint32_t incl = warp_incl(np), sum = __reduce_add_sync(0xFFFFFFFFu, d);
-            const uint32_t pieces = __shfl_sync(0xFFFFFFFFu, incl, 31);
-            const bool fits = pieces <= kSoloPieces && sum <= kSoloEdges;
+            const uint32_t v = lane < m ? B.win_v[lane] : 0u;
+            const uint32_t ab = d > kPiece ? 0x10000u : (d ? 1u : 0u), u = d > kPiece ? pieces_of(d) : 0u;
+            const uint32_t iab = warp_incl(ab), iu = warp_incl(u), sum = __reduce_add_sync(0xFFFFFFFFu, d);
+            const uint32_t all_ab = __shfl_sync(0xFFFFFFFFu, iab, 31), all_u = __shfl_sync(0xFFFFFFFFu, iu, 31);
+            const uint32_t pieces = (all_ab & 0xFFFFu) + all_u;
+            const bool fits = solo && pieces <= kSoloPieces && sum <= kSoloEdges;
+            const uint32_t pab = iab - ab, pu = iu - u;
             if (fits) {
-                uint32_t at = incl - np;
+                uint32_t at = (pab & 0xFFFFu) + pu;
                 for (uint32_t k = 0; k < d; k += kPiece) B.solo[at++] = make_uint4(b + k, min(kPiece, d - k), v, 0u);
+            } else if (pieces) {
+                Span at{0u, 0u, 0u};
+                if (lane == 0) at = reserve(tail, Span{all_ab & 0xFFFFu, all_ab >> 16, all_u});
+                at.a = __shfl_sync(0xFFFFFFFFu, at.a, 0) + (pab & 0xFFFFu);
+                at.b = __shfl_sync(0xFFFFFFFFu, at.b, 0) + (pab >> 16);
+                at.u = __shfl_sync(0xFFFFFFFFu, at.u, 0) + pu;
+                put_entry(a, at, v, b, d);
             }
             if (lane == 0) {
+                if (lvl && m) {
+                    atomicAdd(&lvl[1], (unsigned long long)m);
+                    atomicAdd(&lvl[2], (unsigned long long)sum);
+                }
+                B.win_cnt = 0;
                 B.tot_u[0] = pieces;
                 B.tot_deg[0] = sum;
                 B.ok = fits;
-                if (fits) B.win_cnt = 0;
             }
         }
+        if (lvl) return F;  // (the caller reads nothing of it, and its barrier follows)
         __syncthreads();
-        if (B.ok) return Flushed{B.tot_u[0], m, B.tot_deg[0], true};
-        __syncthreads();  // too many edges: the general way below
+        F.pieces = B.tot_u[0];
+        F.deg = B.tot_deg[0];
+        F.in_solo = B.ok;
+        return F;
     }
     uint32_t ab = 0, u = 0, ed = 0;  // short | long << 16 entries, pieces of the long ones, edges
     for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
