@@ -380,9 +380,10 @@ void attach_tiles(blest_graph* g, const uint32_t* rows, const uint32_t* masks, c
 // The pull side of a resident graph: CSR lists ordered by descending
 // neighbour degree, the has-in-neighbour bitmap and the long-list pieces;
 // then the graph's stream and default workspace.
-// `symmetric`: the caller knows that the tiles' edges are symmetric and the
-// same as the lists'; otherwise that is checked on the device.
-void graph_attach_csr(blest_graph* g, const blest_csr_view* csr, bool symmetric) {
+// `symmetric`: what the caller knows of the tiles' edges: kSymmetric (and the
+// same as the lists'), kDirected, or kUnknown, which is checked on the device.
+enum Symmetry { kDirected, kSymmetric, kUnknown };
+void graph_attach_csr(blest_graph* g, const blest_csr_view* csr, Symmetry symmetric) {
     blest::dev::DevGraph& d = g->d;
     d.nnz = csr->nnz;
     d.degree_total = csr->nnz;
@@ -409,8 +410,10 @@ void graph_attach_csr(blest_graph* g, const blest_csr_view* csr, bool symmetric)
     }
     {
         std::vector<uint32_t> hasIn(((size_t)csr->n + 31) / 32 + 4, 0u);
-        for (uint32_t u = 0; u < csr->n; ++u)
-            if (csr->row_ptrs[u + 1] > csr->row_ptrs[u]) hasIn[u >> 5] |= 1u << (u & 31);
+#pragma omp parallel for schedule(static, 4096)
+        for (int64_t w = 0; w < (int64_t)((csr->n + 31) / 32); ++w)
+            for (uint32_t u = (uint32_t)w * 32; u < std::min(csr->n, (uint32_t)w * 32 + 32); ++u)
+                if (csr->row_ptrs[u + 1] > csr->row_ptrs[u]) hasIn[w] |= 1u << (u & 31);
         d.has_in = blest::upload(g, hasIn.data(), hasIn.size());
     }
     {
@@ -424,7 +427,7 @@ void graph_attach_csr(blest_graph* g, const blest_csr_view* csr, bool symmetric)
         d.pull_chunks = blest::upload(g, chunks.data(), chunks.size());
     }
     g->undirected_edges = csr->nnz / 2;
-    g->symmetric = symmetric || blest::tiles_symmetric_device(d, nullptr);
+    g->symmetric = symmetric == kSymmetric || (symmetric == kUnknown && blest::tiles_symmetric_device(d, nullptr));
     uint64_t out_edges = d.nnz;
     blest::OutLists out;
     if (g->symmetric) {
@@ -498,7 +501,7 @@ int blest_graph_create(const blest_bvss_view* bvss, const blest_csr_view* csr, b
             release();
             (void)d;
         }
-        graph_attach_csr(g, csr, false);
+        graph_attach_csr(g, csr, kUnknown);
         *out = g;
     });
     if (rc != BLEST_OK && g) blest_graph_destroy(g);
@@ -533,7 +536,9 @@ int blest_graph_create_from_csc(const blest_csc* csc, const blest_csc* csr, int 
             throw;
         }
         blest::device_bvss_free(b);
-        graph_attach_csr(g, &cv, csr == nullptr);  // without a CSR: checked above
+        // without a CSR: checked above; in- and out-degrees that differ
+        // somewhere settle it too
+        graph_attach_csr(g, &cv, !csr ? kSymmetric : (c.col_ptrs == t.col_ptrs ? kUnknown : kDirected));
         *out = g;
     });
     if (rc != BLEST_OK && g) blest_graph_destroy(g);

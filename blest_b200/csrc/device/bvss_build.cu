@@ -582,22 +582,26 @@ bool out_lists_device(const dev::DevGraph& d, cudaStream_t s, OutLists& out) {
     BLEST_CUDA(cudaGetDevice(&dev));
     BLEST_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     Scratch tmp;
-    uint32_t* degree = tmp.get<uint32_t>((size_t)d.n + 1);
     unsigned long long* edges = tmp.get<unsigned long long>(1);
-    BLEST_CUDA(cudaMemsetAsync(degree, 0, 4 * ((size_t)d.n + 1), s));
-    BLEST_CUDA(cudaMemsetAsync(edges, 0, 8, s));
-    dev::out_count_kernel<<<sms * 8, 256, 0, s>>>(d, degree, edges);
-    BLEST_CUDA(cudaGetLastError());
-    unsigned long long total = 0;
-    BLEST_CUDA(cudaMemcpyAsync(&total, edges, 8, cudaMemcpyDeviceToHost, s));
-    BLEST_CUDA(cudaStreamSynchronize(s));
-    if (total >= 0xFFFFFF00ull) return false;
     out = OutLists{};
-    out.edges = (uint32_t)total;
     try {
+        // the degrees are counted into `ptrs` and scanned in place
         out.ptrs = dmalloc<uint32_t>((size_t)d.n + 1);
+        BLEST_CUDA(cudaMemsetAsync(out.ptrs, 0, 4 * ((size_t)d.n + 1), s));
+        BLEST_CUDA(cudaMemsetAsync(edges, 0, 8, s));
+        dev::out_count_kernel<<<sms * 8, 256, 0, s>>>(d, out.ptrs, edges);
+        BLEST_CUDA(cudaGetLastError());
+        unsigned long long total = 0;
+        BLEST_CUDA(cudaMemcpyAsync(&total, edges, 8, cudaMemcpyDeviceToHost, s));
+        BLEST_CUDA(cudaStreamSynchronize(s));
+        if (total >= 0xFFFFFF00ull) {
+            cudaFree(out.ptrs);
+            out = OutLists{};
+            return false;
+        }
+        out.edges = (uint32_t)total;
         out.ids = dmalloc<uint32_t>(total);
-        exclusive_scan(degree, out.ptrs, d.n + 1, s);
+        exclusive_scan(out.ptrs, out.ptrs, d.n + 1, s);
         dev::out_fill_kernel<<<sms * 8, 256, 0, s>>>(d, out.ptrs, out.ids);
         BLEST_CUDA(cudaGetLastError());
         BLEST_CUDA(cudaStreamSynchronize(s));
