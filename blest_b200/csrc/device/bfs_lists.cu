@@ -225,11 +225,16 @@ __device__ __forceinline__ void emit(const BfsArgs& a, BlockState& B, const uint
 // The block's buffered discoveries as queue entries: into the global queues
 // (one reservation per block), or, when `solo` and they fit, as pieces into
 // B.solo. Adds the block's discovery count and degree sum to lvl[1], lvl[2]
-// (when lvl).
+// (when lvl). The buffer's counters stay as they are: every warp reads them
+// here, so they are reset behind a barrier that follows (reset_buffer).
 struct Flushed {
     uint32_t pieces, disc, deg;
     bool in_solo;
 };
+__device__ __forceinline__ void reset_buffer(BlockState& B) {  // one thread, between two block barriers
+    B.win_cnt = 0;
+    B.win_end = kWinners;
+}
 __device__ __forceinline__ Flushed flush(const BfsArgs& a, BlockState& B, const Tail& tail, unsigned long long* lvl,
                                          uint32_t disc, uint32_t deg, bool solo) {
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -266,7 +271,6 @@ __device__ __forceinline__ Flushed flush(const BfsArgs& a, BlockState& B, const 
                     atomicAdd(&lvl[1], (unsigned long long)m);
                     atomicAdd(&lvl[2], (unsigned long long)sum);
                 }
-                B.win_cnt = 0;
                 B.tot_u[0] = pieces;
                 B.tot_deg[0] = sum;
                 B.ok = fits;
@@ -321,10 +325,6 @@ __device__ __forceinline__ Flushed flush(const BfsArgs& a, BlockState& B, const 
         if (!F.in_solo) B.base = reserve(tail, Span{all_ab & 0xFFFFu, all_ab >> 16, all_u});
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        B.win_cnt = 0;
-        B.win_end = kWinners;
-    }
     const uint32_t pab = before_ab + iab - ab, pu = before_u + iu - u;
     if (F.in_solo) {
         uint32_t at = (pab & 0xFFFFu) + pu;
@@ -471,8 +471,8 @@ __device__ __forceinline__ void push_level(const BfsArgs& a, BlockState& B, cons
 }
 
 // End of a level (or of a part of it): the grid barrier, then thread 0 reads
-// the level's counters. Adds the block's disc/deg first when `add`. Returns
-// false when the run has an error recorded.
+// the level's counters; the block's buffer is empty again. Adds the block's
+// disc/deg first when `add`. Returns false when the run has an error recorded.
 __device__ __forceinline__ bool level_end(const BfsArgs& a, BlockState& B, unsigned long long* lvl, bool add,
                                           uint32_t disc, uint32_t deg) {
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -486,6 +486,7 @@ __device__ __forceinline__ bool level_end(const BfsArgs& a, BlockState& B, unsig
     }
     __syncthreads();
     if (threadIdx.x == 0) {
+        reset_buffer(B);
         if (add) {
             uint32_t sd = 0, sg = 0;
             for (uint32_t i = 0; i < nw; ++i) {
@@ -566,6 +567,8 @@ __device__ __forceinline__ void solo_levels(const BfsArgs& a, BlockState& B, Run
         }
         ++done;
         const Flushed F = flush(a, B, tail, nullptr, disc, deg, done < kSoloLevels);
+        // flush's last barrier follows every read of the counters
+        if (threadIdx.x == 0) reset_buffer(B);
         s.D2 = s.D1;
         s.G2 = s.G1;
         s.D1 += F.disc;
@@ -962,10 +965,7 @@ __device__ __forceinline__ void lists_run(const BfsArgs& a) {
         s.size = d > kPiece ? Span{0u, 1u, pieces_of(d)} : Span{d ? 1u : 0u, 0u, 0u};
         s.D1 = 1;
         s.G1 = __ldg(&g.csr_ptrs[src + 1]) - __ldg(&g.csr_ptrs[src]);
-        if (threadIdx.x == 0) {
-            B.win_cnt = 0;
-            B.win_end = kWinners;
-        }
+        if (threadIdx.x == 0) reset_buffer(B);
     }
     if (!grid_barrier(c)) return;
 
