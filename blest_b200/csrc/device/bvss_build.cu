@@ -317,7 +317,9 @@ __global__ void tiles_symmetric_kernel(DevGraph g, uint32_t* seen, uint32_t* bad
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     uint64_t count = 0;
     for (uint32_t r = warp; r < g.no_real; r += nwarps) {
-        if (*(volatile uint32_t*)bad) break;
+        // other warps write the flag meanwhile, and lanes need not read the same
+        // value: the warp leaves as one
+        if (__any_sync(0xFFFFFFFFu, *(volatile uint32_t*)bad)) break;
         const uint32_t t1 = __ldg(&g.rset_tile[r + 1]);
         for (uint32_t t = __ldg(&g.rset_tile[r]) + lane; t < t1; t += 32) {
             const uint4 rows = __ldg(&g.row4[t]);
