@@ -903,7 +903,9 @@ __device__ __forceinline__ void heavy_level(const BfsArgs& a, uint64_t hq, uint3
         const uint32_t q1 = min(it.z, q0 + kHeavyChunk);
         uint32_t hitv = kUnreached;
         for (uint32_t base = q0; base < q1 && hitv == kUnreached; base += 32) {
-            if (__ldcg(&a.visited[w]) & b) break;  // another piece found it
+            // another piece found it (lanes need not read the same while
+            // that happens: the warp leaves as one)
+            if (__any_sync(0xFFFFFFFFu, __ldcg(&a.visited[w]) & b)) break;
             const uint32_t idx = base + lane;
             const uint32_t v[1] = {idx < q1 ? __ldg(&g.csr_ids[idx]) : kUnreached};
             const uint32_t hb = __ballot_sync(0xFFFFFFFFu, front.first(v) != kUnreached);
