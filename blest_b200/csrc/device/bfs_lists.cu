@@ -41,6 +41,7 @@
 #include "../host/common.hpp"
 #include "../host/errors.hpp"
 #include "bfs_args.cuh"
+#include "bfs_grid.hpp"
 #include "common.cuh"
 #include "runtime.hpp"
 
@@ -1247,14 +1248,8 @@ void launch_lists(const blest_graph* g, const dev::BfsArgs& args, int blocks_per
         }
     }
     if (maxBlocks < 1) throw Error(BLEST_ERR_CUDA, "BFS kernel cannot be resident with this block size");
-    const int bps = blocks_per_sm > 0 ? std::min(blocks_per_sm, maxBlocks) : maxBlocks;
-    // A small graph takes no more blocks than it has work for (2048 edges or
-    // 512 vertices each), and one block per SM until its levels fill more:
-    // every block costs every barrier (RMAT-16 45.5 us with two per SM, 43.4
-    // with one; RMAT-18 53.5 and 49.8; uniform 2 M vertices 90 and 98).
-    uint64_t work = std::max<uint64_t>(g->d.n / 512, g->d.nnz / 2048) + 1;
-    if (g->d.n < (1u << 20)) work = std::min<uint64_t>(work, (uint64_t)g->sm_count);
-    const int grid = (int)std::min<uint64_t>(cooperative_grid(bps, g->sm_count, grid_cap), work);
+    const int want = bfs_lists_blocks(g->d.n, g->d.nnz, g->sm_count, maxBlocks, blocks_per_sm, threads);
+    const int grid = std::min(want, cooperative_grid(maxBlocks, g->sm_count, grid_cap));
     void* kargs[] = {(void*)&args};
     BLEST_CUDA(cudaLaunchCooperativeKernel((void*)kern, grid, threads, kargs, smem, s));
 }
