@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
+#include <cstddef>
 #include <cstring>
 #include <thread>
 #include <string>
@@ -145,29 +146,41 @@ void workspace_alloc(const blest_graph* g, Workspace& w) {
     };
     alloc((void**)&w.visited, 4ull * w.words);
     for (int i = 0; i < 3; ++i) alloc((void**)&w.frontier[i], 4ull * w.words);
-    alloc((void**)&w.q_rset, 4ull * w.qcap);
-    alloc((void**)&w.q_off, 4ull * w.qcap);
-    alloc((void**)&w.counters, sizeof(dev::RunCounters));
-    alloc((void**)&w.list_counters, sizeof(dev::RunCounters));
-    alloc((void**)&w.cc_counters, sizeof(dev::RunCounters));
-    BLEST_CUDA(cudaMemset(w.list_counters, 0, sizeof(dev::RunCounters)));
-    BLEST_CUDA(cudaMemset(w.cc_counters, 0, sizeof(dev::RunCounters)));
+    // One array for what no two kernels use at once: the tile queue (BFS over
+    // tiles, label propagation), union-find's words, the queues of BFS over
+    // lists. Each writes what it reads.
+    size_t scratch = std::max(8ull * w.qcap, 8ull * n);
+    if (g->d.out_ptrs) scratch = std::max(scratch, sizeof(uint4) * (size_t)g->d.piece_cap);
+    alloc((void**)&w.q_rset, scratch);
+    w.q_off = w.q_rset + w.qcap;
+    w.cc_parent = w.q_rset;
+    w.pieces = g->d.out_ptrs ? reinterpret_cast<uint4*>(w.q_rset) : nullptr;
+    alloc((void**)&w.counters, 3 * sizeof(dev::RunCounters));
+    w.list_counters = w.counters + 1;
+    w.cc_counters = w.counters + 2;
+    BLEST_CUDA(cudaMemset(w.counters, 0, 3 * sizeof(dev::RunCounters)));
     BLEST_CUDA(cudaStreamSynchronize(nullptr));
     alloc((void**)&w.levels, 4ull * n);
     alloc((void**)&w.parents, 4ull * n);
-    alloc((void**)&w.cc_parent, 8ull * n);
     alloc((void**)&w.trace, sizeof(blest_level_trace) * BLEST_TRACE_CAPACITY);
     summary_geometry(w.words, w.sum_shift, w.sum_words);
     for (int i = 0; i < 3; ++i) alloc((void**)&w.summary[i], 4ull * w.sum_words);
-    if (g->d.out_ptrs) alloc((void**)&w.pieces, sizeof(uint4) * (size_t)g->d.piece_cap);
     w.heavy_cap = g->d.nnz / 1024 + 64;
     alloc((void**)&w.heavy, sizeof(uint4) * w.heavy_cap);
-    BLEST_CUDA(cudaMallocHost((void**)&w.host_counters, sizeof(dev::RunCounters)));
-    BLEST_CUDA(cudaHostAlloc((void**)&w.records, sizeof(dev::RunRecord) * kRecordRing, cudaHostAllocMapped));
-    BLEST_CUDA(cudaHostAlloc((void**)&w.cc_record, sizeof(dev::CcRecord), cudaHostAllocMapped));
+    // pinned: the counters' mirror, the ring of BFS records, union-find's record
+    struct Pinned {
+        dev::RunCounters counters;
+        dev::RunRecord records[kRecordRing];
+        dev::CcRecord cc;
+    };
+    static_assert(offsetof(Pinned, counters) == 0, "workspace_free frees it by the counters");
+    Pinned* pinned = nullptr;
+    BLEST_CUDA(cudaHostAlloc((void**)&pinned, sizeof(Pinned), cudaHostAllocMapped));
+    w.host_counters = &pinned->counters;
+    w.records = pinned->records;
+    w.cc_record = &pinned->cc;
     // no slot may look like a finished call before its kernel wrote it
-    std::memset((void*)w.cc_record, 0xFF, sizeof(dev::CcRecord));
-    std::memset((void*)w.records, 0xFF, sizeof(dev::RunRecord) * kRecordRing);
+    std::memset((void*)pinned, 0xFF, sizeof(Pinned));
     w.call_slot = new int8_t[kRecordRing];
     BLEST_CUDA(cudaEventCreate(&w.ev_start));
     BLEST_CUDA(cudaEventCreate(&w.ev_stop));
@@ -177,20 +190,13 @@ void workspace_free(Workspace& w) {
     cudaFree(w.visited);
     for (auto& f : w.frontier) cudaFree(f);
     cudaFree(w.q_rset);
-    cudaFree(w.q_off);
     cudaFree(w.counters);
-    cudaFree(w.list_counters);
-    cudaFree(w.cc_counters);
     cudaFree(w.levels);
     cudaFree(w.parents);
-    cudaFree(w.cc_parent);
     cudaFree(w.trace);
     for (auto& x : w.summary) cudaFree(x);
-    cudaFree(w.pieces);
     cudaFree(w.heavy);
     mbfs_scratch_free(w.mbfs);
-    if (w.records) cudaFreeHost(w.records);
-    if (w.cc_record) cudaFreeHost(w.cc_record);
     delete[] w.call_slot;
     cudaFree(w.levels_b);
     cudaFree(w.parents_b);
@@ -443,7 +449,7 @@ void graph_attach_csr(blest_graph* g, const blest_csr_view* csr, Symmetry symmet
     }
     if (d.out_ptrs) {
         uint4* heads = blest::dev_alloc<uint4>(g, csr->n);
-        blest::list_heads_device(d, heads, nullptr);
+        blest::list_heads_device(d, heads, nullptr);  // done when workspace_alloc returns
         d.heads = heads;
     }
     d.piece_cap = (uint32_t)(csr->n + out_edges / blest::dev::kBfsPieceEdges + 64);

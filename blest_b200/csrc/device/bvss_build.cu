@@ -576,7 +576,6 @@ void list_heads_device(const dev::DevGraph& d, uint4* heads, cudaStream_t s) {
     BLEST_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     dev::list_heads_kernel<<<sms * 8, 256, 0, s>>>(d, heads);
     BLEST_CUDA(cudaGetLastError());
-    BLEST_CUDA(cudaStreamSynchronize(s));
 }
 
 bool out_lists_device(const dev::DevGraph& d, cudaStream_t s, OutLists& out) {

@@ -30,9 +30,10 @@ struct Workspace {
     uint32_t qcap = 0;         // queue capacity (entries)
     uint32_t* visited = nullptr;
     uint32_t* frontier[3] = {nullptr, nullptr, nullptr};
+    // q_rset, q_off, cc_parent and pieces share one array (workspace_alloc).
     uint32_t* q_rset = nullptr;
     uint32_t* q_off = nullptr;
-    dev::RunCounters* counters = nullptr;
+    dev::RunCounters* counters = nullptr;       // and the next two: one array
     dev::RunCounters* list_counters = nullptr;  // BFS over lists: zero between runs
     dev::RunCounters* cc_counters = nullptr;    // union-find: the same
     dev::CcRecord* cc_record = nullptr;         // union-find: the last run's outcome (mapped host memory)
@@ -178,7 +179,7 @@ struct OutLists {
     uint32_t* ids = nullptr;
     uint32_t edges = 0;
 };
-// DevGraph::heads of the pull lists.
+// DevGraph::heads of the pull lists (not waited for).
 void list_heads_device(const dev::DevGraph& d, uint4* heads, cudaStream_t s);
 bool out_lists_device(const dev::DevGraph& d, cudaStream_t s, OutLists& out);
 void mbfs_scratch_free(void* p);
