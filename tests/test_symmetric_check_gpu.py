@@ -68,3 +68,25 @@ def test_hub_sets(gpu):
     check(from_pairs(n, np.concatenate([a, b]), np.concatenate([b, a])))
     # the same with one hub's edges turned one way
     check(from_pairs(n, np.concatenate([a, b[a != 5]]), np.concatenate([b, a[a != 5]])))
+
+
+@pytest.mark.parametrize("to_hub", [False, True])
+@pytest.mark.parametrize("lists", ["transpose", "same"])
+def test_one_direction_of_one_edge(gpu, to_hub, lists):
+    """One edge between a hub and a leaf of its own lacks its reverse. With the
+    out-lists passed as pull lists (which describe the same edges then, but the
+    wrong way) only the missing reverse tells; components read the tiles."""
+    n = 5000
+    src, dst = symmetric_pairs(n - 1, 20_000, 13)
+    hub_src = np.append(src, np.full(1500, 7))
+    hub_dst = np.append(dst, np.arange(100, 1600))
+    both = (np.append(hub_src, np.arange(100, 1600)), np.append(hub_dst, np.full(1500, 7)))
+    one = (n - 1, 7) if to_hub else (7, n - 1)
+    csc = from_pairs(n, np.append(both[0], one[0]), np.append(both[1], one[1]))
+    g = Graph(Bvss.build(csc), csc if lists == "same" else csc.transpose())
+    labels, _ = g.cc()
+    np.testing.assert_array_equal(labels, O.cc_csc(csc.n, csc.col_ptrs, csc.rows))
+    if lists == "transpose":
+        for s in (7, n - 1, 0):
+            lv, _, _ = g.bfs(s)
+            np.testing.assert_array_equal(lv, O.bfs_csc(csc.n, csc.col_ptrs, csc.rows, s))
