@@ -465,6 +465,8 @@ __device__ __forceinline__ void cc_union_run(const CcUnionArgs& a) {
         if (threadIdx.x == 0) {
             const bool ok = (barrier_arrive_wait(c) & kArriveError) == 0;
             s_hooked = ok ? ld_relaxed64(&hooked[round]) : ~0ull;
+            // passes over edges: A, the rounds so far, D
+            if (blockIdx.x == 0) c->iterations = g.nnz ? round + 3 : 0;
         }
         __syncthreads();
         const uint64_t h = s_hooked;
@@ -567,7 +569,6 @@ __device__ __forceinline__ void cc_union_run(const CcUnionArgs& a) {
         const uint32_t r = parent[v];
         if (r != v) a.labels[v] = a.labels[r];
     }
-    if (tid == 0) c->iterations = g.nnz ? 2 : 0;  // two phases read the edges (A and D)
 }
 
 __global__ void __launch_bounds__(512, 3) cc_union_kernel(CcUnionArgs a) {

@@ -82,7 +82,7 @@ struct RunCounters {
     unsigned int levels;            // last level with discoveries
     unsigned int push_levels;
     unsigned int pull_levels;
-    unsigned int iterations;        // CC: label-propagation iterations
+    unsigned int iterations;        // CC: label-propagation iterations, or union-find's passes over edges
     unsigned int trace_records;     // multi-source BFS: level records written (0: BFS counts by levels)
     unsigned int pad[6];
     // Slots reused across levels/iterations (queue counters, heavy-list

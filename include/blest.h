@@ -373,15 +373,18 @@ int blest_selftest_barrier(uint32_t blocks, uint32_t missing_blocks, uint64_t ti
 /* ---- connected components ------------------------------------------------ */
 /* Mirrors CCResult (CC/CCKernel.cuh:21-26). */
 typedef struct blest_cc_stats {
-    double time;
+    double time;             /* seconds on the device: of the one kernel by its own clock
+                                (symmetric graphs), or between events around the launches */
     uint32_t no_components;
-    uint32_t iterations;
+    uint32_t iterations;     /* passes over edges, 0 without edges. Symmetric graphs: union-find's
+                                (sampling, hooking rounds, linking: 3 to 14, by how the threads
+                                meet, so two runs may differ); else label propagation's */
 } blest_cc_stats;
-/* CCKernel::hostCode() (CC/BVSSCCKernel.cuh:1067-1311): min-label
- * propagation to its fixpoint. labels_out[v] = the smallest vertex id that
- * reaches v, i.e. the minimum id of v's component on a symmetric graph
- * (the kernel's result before the reference's host relabel, which is
- * offered separately by blest_cc_relabel_dense). */
+/* CCKernel::hostCode() (CC/BVSSCCKernel.cuh:1067-1311). labels_out[v] = the
+ * smallest vertex id that reaches v, i.e. the minimum id of v's component on
+ * a symmetric graph (the kernel's result before the reference's host relabel,
+ * which is offered separately by blest_cc_relabel_dense): by union-find on
+ * symmetric graphs, by min-label propagation to its fixpoint on others. */
 int blest_cc(blest_graph* g, uint32_t* labels_out, int out_mem, blest_cc_stats* stats);
 int blest_cc_ws(blest_workspace* ws, uint32_t* labels_out, int out_mem, void* stream, blest_cc_stats* stats);
 /* Host relabel to dense ids 0..k-1 in order of the minimum id, as
