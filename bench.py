@@ -130,7 +130,8 @@ def reached_edges(csr_degrees: np.ndarray, levels: np.ndarray) -> int:
 
 def algorithmic_bytes(bvss_arrays: dict, levels: np.ndarray) -> int:
     """5*S_R + 12*V_R + 4*N_R: slices/vsets of rsets holding a reached vertex,
-    plus one 4-byte level per reached vertex."""
+    plus one 4-byte level per reached vertex: one pass over the tiles, as the
+    kernel of the b1-MMA slice test reads them."""
     reached = np.nonzero(levels != 0xFFFFFFFF)[0]
     rsets = np.unique(reached >> 3)
     rp = bvss_arrays["real_ptrs"]
@@ -138,6 +139,27 @@ def algorithmic_bytes(bvss_arrays: dict, levels: np.ndarray) -> int:
     v_r = int((rp[rsets + 1].astype(np.int64) - rp[rsets]).sum())
     s_r = int((ssp[rp[rsets + 1]].astype(np.int64) - ssp[rp[rsets]].astype(np.int64)).sum())
     return 5 * s_r + 12 * v_r + 4 * reached.size
+
+
+def list_bytes(levels: np.ndarray) -> int:
+    """12*N_R: what BFS over lists cannot do without, a list bound and one edge
+    read and a level written per reached vertex."""
+    return 12 * int((levels != 0xFFFFFFFF).sum())
+
+
+def bfs_roofline(over_lists: bool, algo_bytes: float, launch_s: float, traffic, peak: float, peak_kind: str) -> dict:
+    """Roofline entry of a BFS line. Over tiles the bound is HBM and the bytes
+    one pass over them. Over lists no unit is near its peak (chains of dependent
+    reads, scattered L1 accesses): achieved is the least traffic over the time,
+    and the DRAM share comes from the captured traffic, where there is one."""
+    achieved = algo_bytes / launch_s / 1e9
+    line = {"bound": "latency" if over_lists else "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
+            "frac": round(achieved / peak, 4), "peak_source": peak_kind, "traffic": traffic if over_lists else None,
+            "algorithmic_bytes_per_launch": int(algo_bytes), "avg_launch_ms": round(launch_s * 1e3, 4)}
+    if over_lists and traffic:
+        line["dram_gbs"] = round(traffic / launch_s / 1e9, 1)
+        line["dram_frac"] = round(traffic / launch_s / 1e9 / peak, 4)
+    return line
 
 
 # ----------------------------------------------------------------- clocks
@@ -974,6 +996,7 @@ def run_b200(args, rank, world):
     host_lv = np.empty(n, dtype=np.uint32)
     mr, algo = [], []
     arrays = bvss.arrays()
+    over_lists = (tuned["slice_test"] if tuned else args.slice_test) != "mma"
     check = rank == 0 and not args.skip_check
     parity = {"sources_checked": 0, "mismatches": 0, "against": "oracle bfs_omp (oracle/oracle.c), all sources"}
     cpu_secs, cpu_edges, cpu_used = 0.0, 0, 0
@@ -982,7 +1005,7 @@ def run_b200(args, rank, world):
     for s in sources:
         ws.bfs(int(s), host_lv, sptr, params=params)
         mr.append(reached_edges(deg, host_lv))
-        algo.append(algorithmic_bytes(arrays, host_lv))
+        algo.append(list_bytes(host_lv) if over_lists else algorithmic_bytes(arrays, host_lv))
         if check:
             t = time.perf_counter()
             want, cpu_used = O.bfs_omp(n, csc.col_ptrs, csc.rows, csr.col_ptrs, csr.rows, int(s), 0)
@@ -1124,10 +1147,7 @@ def run_b200(args, rank, world):
                 log(f"[trace]   L{r.level:<4d} {'push' if r.direction == 1 else 'pull'} frontier {r.frontier:>9d} "
                     f"units {r.work_units:>10d} {(nx.start_ns - r.start_ns) / 1e3:9.1f} us{sweep}")
     peak, peak_kind = measured_peak()
-    avg_bytes = float(np.mean(algo))
     avg_launch_s = float(np.mean(bfs_ms)) * 1e-3
-    achieved = avg_bytes / avg_launch_s / 1e9
-    traffic = profiled_traffic(args.workload)
     result = {
         "metric": "BFS GTEPS (single-source, direction-optimising BVSS BFS)",
         "value": round(value, 3), "unit": "GTEPS", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
@@ -1148,10 +1168,8 @@ def run_b200(args, rank, world):
                 "d2h_gbs_measured": round(d2h_gbs, 2), "copy_bound_gteps": round(copy_bound, 3),
                 "frac_of_copy_bound": round(e2e / world / copy_bound, 3)},
         "gpu_launches": int(len(sources)) * args.steps,
-        "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-                     "frac": round(achieved / peak, 4), "peak_source": peak_kind,
-                     "traffic": traffic, "algorithmic_bytes_per_launch": int(avg_bytes),
-                     "avg_launch_ms": round(avg_launch_s * 1e3, 4)},
+        "roofline": bfs_roofline(over_lists, float(np.mean(algo)), avg_launch_s, profiled_traffic(args.workload),
+                                 peak, peak_kind),
     }
     if check:
         result["parity"] = parity
@@ -1164,7 +1182,8 @@ def run_b200(args, rank, world):
 
 
 def run_cc(args, rank, world):
-    """Connected components by BVSS label propagation: ms per full CC run
+    """Connected components (union-find: the workloads' graphs are symmetric):
+    ms per full CC run
     (labels = minimum vertex id of the component), device output; e2e adds
     the labels' device->host copy into pinned memory."""
     import torch
