@@ -53,6 +53,19 @@ T* upload(blest_graph* g, const T* src, size_t count) {
     return d;
 }
 
+// Runs f; false when device memory did not suffice (f leaves nothing behind).
+template <class F>
+bool when_it_fits(F f) {
+    try {
+        f();
+        return true;
+    } catch (const Error& e) {
+        if (e.code != BLEST_ERR_OOM) throw;
+        cudaGetLastError();  // else the next launch's check finds it
+        return false;
+    }
+}
+
 void validate_csr(const blest_csr_view* c);
 
 // Structural checks the kernels rely on for memory safety (every index
@@ -136,7 +149,9 @@ void summary_geometry(uint32_t words, uint32_t& shift, uint32_t& sum_words) {
     }
 }
 
-void workspace_alloc(const blest_graph* g, Workspace& w) {
+namespace {
+// `over_lists`: with the queues of BFS over lists.
+void workspace_fill(const blest_graph* g, Workspace& w, bool over_lists) {
     const uint32_t n = g->d.n;
     w.words = (((n + 31) / 32) + 3) & ~3u;
     w.qcap = g->d.no_real * 8 + 64;
@@ -150,11 +165,11 @@ void workspace_alloc(const blest_graph* g, Workspace& w) {
     // tiles, label propagation), union-find's words, the queues of BFS over
     // lists. Each writes what it reads.
     size_t scratch = std::max(8ull * w.qcap, 8ull * n);
-    if (g->d.out_ptrs) scratch = std::max(scratch, sizeof(uint4) * (size_t)g->d.piece_cap);
+    if (over_lists) scratch = std::max(scratch, sizeof(uint4) * (size_t)g->d.piece_cap);
     alloc((void**)&w.q_rset, scratch);
     w.q_off = w.q_rset + w.qcap;
     w.cc_parent = w.q_rset;
-    w.pieces = g->d.out_ptrs ? reinterpret_cast<uint4*>(w.q_rset) : nullptr;
+    w.pieces = over_lists ? reinterpret_cast<uint4*>(w.q_rset) : nullptr;
     alloc((void**)&w.counters, 3 * sizeof(dev::RunCounters));
     w.list_counters = w.counters + 1;
     w.cc_counters = w.counters + 2;
@@ -184,6 +199,14 @@ void workspace_alloc(const blest_graph* g, Workspace& w) {
     w.call_slot = new int8_t[kRecordRing];
     BLEST_CUDA(cudaEventCreate(&w.ev_start));
     BLEST_CUDA(cudaEventCreate(&w.ev_stop));
+}
+}  // namespace
+
+void workspace_alloc(const blest_graph* g, Workspace& w) {
+    // (what fits only without the list queues gets none: its BFS goes over tiles)
+    if (g->d.out_ptrs && when_it_fits([&] { workspace_fill(g, w, true); })) return;
+    workspace_free(w);
+    workspace_fill(g, w, false);
 }
 
 void workspace_free(Workspace& w) {
@@ -433,31 +456,51 @@ void graph_attach_csr(blest_graph* g, const blest_csr_view* csr, Symmetry symmet
         d.pull_chunks = blest::upload(g, chunks.data(), chunks.size());
     }
     g->undirected_edges = csr->nnz / 2;
-    g->symmetric = symmetric == kSymmetric || (symmetric == kUnknown && blest::tiles_symmetric_device(d, nullptr));
+    g->symmetric = symmetric == kSymmetric;
+    if (symmetric == kUnknown)
+        blest::when_it_fits([&] { g->symmetric = blest::tiles_symmetric_device(d, nullptr); });
+    // What BFS over lists adds to the graph: out-lists of its own, if directed,
+    // and the heads. A graph that fits only without them does without them (its
+    // BFS goes over tiles).
+    const size_t kept = g->allocations.size();
+    const uint64_t kept_bytes = g->graph_bytes;
+    auto without_lists = [&] {
+        for (; g->allocations.size() > kept; g->allocations.pop_back()) cudaFree(g->allocations.back());
+        g->graph_bytes = kept_bytes;
+        d.out_ptrs = d.out_ids = nullptr;
+        d.heads = nullptr;
+    };
     uint64_t out_edges = d.nnz;
-    blest::OutLists out;
-    if (g->symmetric) {
-        d.out_ptrs = d.csr_ptrs;
-        d.out_ids = d.csr_ids;
-    } else if (blest::out_lists_device(d, nullptr, out)) {
-        g->allocations.push_back(out.ptrs);
-        g->allocations.push_back(out.ids);
-        g->graph_bytes += 4ull * (csr->n + 1ull) + 4ull * out.edges;
-        d.out_ptrs = out.ptrs;
-        d.out_ids = out.ids;
-        out_edges = out.edges;
-    }
-    if (d.out_ptrs) {
-        uint4* heads = blest::dev_alloc<uint4>(g, csr->n);
-        blest::list_heads_device(d, heads, nullptr);  // done when workspace_alloc returns
-        d.heads = heads;
-    }
+    const bool fit = blest::when_it_fits([&] {
+        blest::OutLists out;
+        if (g->symmetric) {
+            d.out_ptrs = d.csr_ptrs;
+            d.out_ids = d.csr_ids;
+        } else if (blest::out_lists_device(d, nullptr, out)) {
+            g->allocations.push_back(out.ptrs);
+            g->allocations.push_back(out.ids);
+            g->graph_bytes += 4ull * (csr->n + 1ull) + 4ull * out.edges;
+            d.out_ptrs = out.ptrs;
+            d.out_ids = out.ids;
+            out_edges = out.edges;
+        }
+        if (d.out_ptrs) {
+            uint4* heads = blest::dev_alloc<uint4>(g, csr->n);
+            blest::list_heads_device(d, heads, nullptr);  // done when workspace_alloc returns
+            d.heads = heads;
+        }
+    });
+    if (!fit) without_lists();
     d.piece_cap = (uint32_t)(csr->n + out_edges / blest::dev::kBfsPieceEdges + 64);
     BLEST_CUDA(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
     g->owns_stream = true;
     g->default_ws = new blest_workspace;
     g->default_ws->g = g;
-    blest::workspace_alloc(g, g->default_ws->w);
+    if (!blest::when_it_fits([&] { blest::workspace_alloc(g, g->default_ws->w); })) {
+        blest::workspace_free(g->default_ws->w);
+        without_lists();
+        blest::workspace_alloc(g, g->default_ws->w);
+    }
 }
 
 }  // namespace
@@ -654,7 +697,7 @@ int blest_bfs_ws(blest_workspace* ws, uint32_t source, uint32_t* levels_out, uin
         uint32_t* dl = out_mem == BLEST_MEM_DEVICE ? levels_out : hl;
         uint32_t* dp = parents_out ? (out_mem == BLEST_MEM_DEVICE ? parents_out : hp) : nullptr;
         // the kernel over tiles leaves its record before its last block has left
-        const bool polled = out_mem == BLEST_MEM_DEVICE && g->d.out_ptrs && p.slice_test != BLEST_TEST_B1_MMA;
+        const bool polled = out_mem == BLEST_MEM_DEVICE && w.pieces && p.slice_test != BLEST_TEST_B1_MMA;
         w.call_slot[seq % blest::kRecordRing] =
             pipelined ? (int8_t)slot : (polled ? blest::kCallPolled : blest::kCallStream);
         blest::launch_bfs(g, w, source, dl, dp, p, s, seq);

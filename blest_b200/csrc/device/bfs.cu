@@ -1004,7 +1004,7 @@ void launch_bfs(const blest_graph* g, Workspace& w, uint32_t src, uint32_t* leve
     if (threads % 32 || threads > 512) throw Error(BLEST_ERR_INVALID_ARG, "threads_per_block must be a multiple of 32, <= 512");
     const bool mma = p.slice_test == BLEST_TEST_B1_MMA;
     w.trace_seq = -1;
-    if (!mma && g->d.out_ptrs) {
+    if (!mma && w.pieces) {  // (else 2^32 - 256 out-edges or more, or no memory for lists)
         a.pieces = w.pieces;
         a.ctr = w.list_counters;
         w.trace_seq = (int64_t)seq;
