@@ -27,10 +27,10 @@
 // shared memory and appends them with one atomic, and while the frontier is
 // small ("solo" levels) block 0 runs the levels alone out of shared memory,
 // with block barriers only, while the others wait in one grid barrier.
-// Against the kernel over tiles (a whole call): RMAT 2^10 63 -> 49 us, RMAT-16
-// 72 -> 64, RMAT-22 215 -> 158 a BFS, grid 2901 x 2801 3080 -> 1200 (widest
-// level, 306 k vertices: 71 -> 24; smallest levels 8 -> 3), uniform 2 M
-// vertices x degree 32 211 -> 137 (41 k-vertex level 62 -> 28).
+// Against the kernel over tiles (a whole call): RMAT 2^10 63 -> 42 us, RMAT-16
+// 72 -> 53, RMAT-22 215 -> 129 a BFS, grid 2901 x 2801 3080 -> 1090 (widest
+// level, 306 k vertices: 71 -> 20; smallest levels 8 -> 3), uniform 2 M
+// vertices x degree 32 211 -> 103 (41 k-vertex level 62 -> 26).
 #include <cuda_runtime.h>
 
 #include <algorithm>
