@@ -696,8 +696,10 @@ int blest_bfs_ws(blest_workspace* ws, uint32_t source, uint32_t* levels_out, uin
         uint32_t* hp = slot ? w.parents_b : w.parents;
         uint32_t* dl = out_mem == BLEST_MEM_DEVICE ? levels_out : hl;
         uint32_t* dp = parents_out ? (out_mem == BLEST_MEM_DEVICE ? parents_out : hp) : nullptr;
-        // the kernel over tiles leaves its record before its last block has left
-        const bool polled = out_mem == BLEST_MEM_DEVICE && w.pieces && p.slice_test != BLEST_TEST_B1_MMA;
+        // The kernel over tiles leaves its record before its last block has left;
+        // and after an asynchronous call the caller may have put work of their
+        // own on the stream, which a sync has always waited for.
+        const bool polled = !async && out_mem == BLEST_MEM_DEVICE && w.pieces && p.slice_test != BLEST_TEST_B1_MMA;
         w.call_slot[seq % blest::kRecordRing] =
             pipelined ? (int8_t)slot : (polled ? blest::kCallPolled : blest::kCallStream);
         blest::launch_bfs(g, w, source, dl, dp, p, s, seq);

@@ -58,7 +58,8 @@ struct Workspace {
     // directly, so reading a finished call's record needs no copy.
     dev::RunRecord* records = nullptr;
     // Of each call (same ring positions): its pipelined slot (0/1), kCallPolled
-    // (done when its record is there) or kCallStream (when its stream is).
+    // (blocking: done when its record is there) or kCallStream (when its stream
+    // is).
     int8_t* call_slot = nullptr;
     // Second level/parent buffers of the pipelined host-output mode (the
     // first pair is `levels`/`parents`), allocated on first use.

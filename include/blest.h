@@ -301,7 +301,8 @@ int blest_bfs_ws(blest_workspace* ws, uint32_t source, uint32_t* levels_out, uin
                  const blest_bfs_params* params, void* stream, int async, blest_bfs_stats* stats);
 #define BLEST_BFS_RECORD_RING 1024
 /* Settle every pending asynchronous call on `ws`: wait for it (and its host
- * copy), check its record; returns the first failure among them, stats =
+ * copy; with device output the last call's stream is waited for, work put on
+ * it since included), check its record; returns the first failure among them, stats =
  * the last call's outcome (time = its kernel's device time). */
 int blest_workspace_sync(blest_workspace* ws, blest_bfs_stats* stats);
 /* Settle only the oldest pending call (so later calls keep running and
