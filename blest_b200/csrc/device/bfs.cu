@@ -1,8 +1,9 @@
 // Single-source direction-optimising BFS over BVSS tiles (push) and CSR
 // in-neighbour lists (pull), as ONE persistent cooperative kernel per BFS: the
-// kernel of the b1-MMA slice test and of blest_bfs_noalloc, whose callers
-// hand over tiles and no out-lists. Every other call pushes over out-lists
-// (bfs_lists.cu), which is faster at every size measured there.
+// kernel of the b1-MMA slice test, of blest_bfs_noalloc, whose callers hand
+// over tiles and no out-lists, and of graphs and workspaces that have no room
+// for lists (or 2^32 - 256 out-edges and more). Every other call pushes over
+// out-lists (bfs_lists.cu), which is faster at every size measured there.
 //
 // Replaces the six BFS kernels of BFS/BVSSBFSKernel.cuh (:33-1261) and the
 // launcher BVSSBFSKernel::hostCode (:1283-1608). Results are the same

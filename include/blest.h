@@ -241,7 +241,8 @@ int blest_workspace_set_grid(blest_workspace* ws, uint32_t blocks);
 #define BLEST_DIR_AUTO 0       /* direction-optimising (push <-> pull) */
 #define BLEST_DIR_PUSH 1       /* top-down only (out-lists; BVSS tiles with the MMA test) */
 #define BLEST_DIR_PULL 2       /* bottom-up over CSR only (after level 1) */
-#define BLEST_TEST_CUDA_CORE 0 /* no slice test: push reads the frontier's out-lists */
+#define BLEST_TEST_CUDA_CORE 0 /* no slice test: push reads the frontier's out-lists (where device memory
+                                  has no room for them: tiles, mask byte & frontier byte) */
 #define BLEST_TEST_B1_MMA 1    /* push over tiles, slice test: mma.sync m8n8k128 b1 AND+POPC (Common.cuh:57-66) */
 typedef struct blest_bfs_params {
     int direction;            /* BLEST_DIR_* */
